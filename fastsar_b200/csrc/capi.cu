@@ -47,7 +47,17 @@ struct DevLevel {
     float *tk = nullptr, *tp = nullptr;
     float2 *phase = nullptr;
     double kc;
+    // how the level runs (plan_forms): LevelForm, and for the two-pass forms the parents and the output columns of one
+    // launch pair (its intermediate fits the workspace's scratch)
+    int form = 0, nn = 0, nj = 0;
+    double cycles = 0.0;              // the largest rotation phase (cycles at the band's edge; level_cycles)
 };
+
+// A level on the float32 CUDA-core kernel, on the one-pass tensor-core kernel, or in two passes through an intermediate
+// of float16 (the mixed-precision form) or float32 (the float32 form).
+enum LevelForm { LV_FP32 = 0, LV_ONE_PASS = 1, LV_TWO_PASS_F16 = 2, LV_TWO_PASS_F32 = 3 };
+
+inline bool two_pass(const DevLevel &v) { return v.form == LV_TWO_PASS_F16 || v.form == LV_TWO_PASS_F32; }
 
 size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
@@ -118,6 +128,7 @@ struct ffbp_plan {
     float4 *seeds = nullptr;          // the float16 tensor-core final stage's ramp seeds [ntiles, Pf]
     int2 *first = nullptr;
     size_t bufA = 0, bufB = 0;
+    size_t scratch = 0;               // bytes of the two-pass levels' intermediate
     std::vector<void *> owned;
     // the host-memory pipeline of ffbp_form_host, made at its first call: an upload and a download stream, per
     // device buffer pair b the events "history b uploaded", "image b formed", "image b downloaded", and a pinned
@@ -174,6 +185,87 @@ struct ffbp_plan {
 };
 
 namespace {
+
+// The largest intermediate of a two-pass level that the float32 form keeps at once: larger levels run in several launch
+// pairs (parents, or columns of one parent), so that a plan needs little more workspace than its level outputs.
+constexpr size_t Y_BYTES = size_t(2) << 30;
+
+// The parents and columns of one launch pair whose intermediate (es bytes a sample) fits `limit`; false when 128 columns
+// of one parent do not.
+bool two_pass_chunk(DevLevel &v, size_t es, size_t limit)
+{
+    const size_t col = (size_t)v.C * v.P * es, par = col * ((v.Ko + 3) & ~3);
+    if (par <= limit) {
+        const int most = (int)std::min<size_t>(limit / par, (size_t)v.Np), n = (v.Np + most - 1) / most;
+        v.nn = (v.Np + n - 1) / n;
+        v.nj = v.Ko;
+        return true;
+    }
+    const int most = (int)(limit / col) & ~127;
+    if (most < 128) return false;
+    const int n = (v.Ko + most - 1) / most;
+    v.nn = 1;
+    v.nj = std::min(most, ((v.Ko + n - 1) / n + 127) & ~127);
+    return true;
+}
+
+// The largest rotation phase of a level, in cycles at the edge of its band, over the children of the first, middle and
+// last parent seen from the first, middle and last pulse.
+double level_cycles(const ffbp_level_desc &L, int B, double kc)
+{
+    const int ns[3] = {0, B / 2, B - 1}, ps[3] = {0, L.P / 2, L.P - 1};
+    double most = 0.0;
+    auto dist = [](const double *a, const double *b) {
+        return std::sqrt((a[0] - b[0]) * (a[0] - b[0]) + (a[1] - b[1]) * (a[1] - b[1]) + (a[2] - b[2]) * (a[2] - b[2]));
+    };
+    for (int n : ns)
+        for (int p : ps) {
+            const double *a = L.h_ant + 3 * (size_t)p;
+            const double r = L.h_range ? L.h_range[p] : dist(L.h_ref + 3 * (size_t)n, a);
+            for (int c = 0; c < L.C; ++c)
+                most = std::max(most, std::fabs(dist(L.h_cen + 3 * ((size_t)n * L.C + c), a) - r));
+        }
+    return most * 2.0 * L.df / ffbp::C_LIGHT * kc;
+}
+
+// The float32 form's levels of larger phases stay on the CUDA-core kernel. That kernel turns every sample by a float32
+// phase in cycles that is taken to radians, an error of about 1e-7 per cycle of rms phase, which the tensor-core level
+// does not make; past about 170 cycles (rms 110) the two differ by more than 1.5e-5 of the image (measured: 9e-6 at 160
+// cycles, 1.8e-5 at 195, 2.7e-5 at 317, 1.2e-4 at 1,870), and a plan's image is to stay what it was to 2e-5.
+constexpr double TC_F32_CYCLES = 170.0;
+
+// How each level runs, and the scratch of the two-pass ones. float32 form: two passes through a float32 intermediate
+// where the shape is covered and the phases are small. FFBP_LEVELS_TC: in one pass, or with FFBP_LEVELS_TC2 (and for shapes the one-pass kernel
+// does not cover) in two through a float16 intermediate; shapes that form does not cover stay in float32. A plan whose
+// level outputs fit the static workspace keeps its scratch inside it too (ffbp_form_static).
+void plan_forms(ffbp_plan *p)
+{
+    const size_t base = 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2));
+    size_t f16 = 0;
+    for (auto &v : p->lv) {
+        const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
+        v.form = LV_FP32;
+        if (!(p->final_mode & FFBP_LEVELS_TC)) continue;
+        if (!(p->final_mode & FFBP_LEVELS_TC2) && ffbp::level_fused_supported(v.C, Lk, v.Dk, Lp, v.Dp)) v.form = LV_ONE_PASS;
+        else if (ffbp::level_tc_supported(v.C, Lk, v.Dk)) {
+            v.form = LV_TWO_PASS_F16;
+            v.nn = v.Np;
+            v.nj = v.Ko;
+            f16 = std::max(f16, ffbp::level_tc_scratch_bytes(v.Np, v.C, v.P, v.Ko));
+        }
+    }
+    const size_t limit = base + align256(f16) <= FFBP_STATIC_WS_BYTES ? FFBP_STATIC_WS_BYTES - base : std::max(f16, Y_BYTES);
+    p->scratch = f16;
+    for (auto &v : p->lv) {
+        const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
+        if (!(p->final_mode & FFBP_LEVELS_TC) && !(v.cycles <= TC_F32_CYCLES)) continue;
+        if (v.form != LV_FP32 || (Lp + v.Dp - 1) / v.Dp > 16 || !two_pass_chunk(v, sizeof(float2), limit) ||
+            !ffbp::level_mma_supported(v.C, Lk, v.Dk, v.nj))
+            continue;
+        v.form = LV_TWO_PASS_F32;
+        p->scratch = std::max(p->scratch, (size_t)v.nn * v.C * v.P * ((v.nj + 3) & ~3) * sizeof(float2));
+    }
+}
 
 const char *const WAIT_MSG = "a tensor-core kernel stopped waiting on its pipeline (a bounded wait ran out) and "
                              "left its output incomplete";
@@ -303,12 +395,14 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
         e = ffbp::launch_phases((const double *)dant, L.P, (const double *)dref, B, (const double *)dcen, L.C,
                                 (const double *)drange, k0c, k1, cancel_free ? 1 : 0, v.phase, s);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "phases kernel"));
+        v.cycles = level_cycles(L, B, v.kc);
         const size_t outn = (size_t)B * L.C * L.Po * L.Ko;
         if (l % 2 == 0) p->bufA = std::max(p->bufA, outn); else p->bufB = std::max(p->bufB, outn);
         p->lv.push_back(v);
         B *= L.C;
     }
     p->ntiles = B;
+    plan_forms(p);
     const ffbp_level_desc &last = d->levels[d->nlev - 1];
     if (p->Pf != last.Po || p->Qf != last.Ko) return cleanup(fail(FFBP_E_ARG, "final stage %dx%d != last level output %dx%d", p->Pf, p->Qf, last.Po, last.Ko));
     if (d->partial ? (long)B * d->T * d->T > (long)d->Nx * d->Ny : (long)B * d->T * d->T != (long)d->Nx * d->Ny)
@@ -354,42 +448,10 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
     return cleanup(FFBP_OK);
 }
 
-// How level l runs: 0 the float32 kernel; 1 the one-pass tensor-core kernel (FFBP_LEVELS_TC, a shape it covers,
-// FFBP_LEVELS_TC2 not set); 2 the two-pass tensor-core kernels (FFBP_LEVELS_TC2, or a shape only they cover).
-static int level_form(const ffbp_plan *p, int l)
-{
-    if (!(p->final_mode & FFBP_LEVELS_TC)) return 0;
-    const DevLevel &v = p->lv[l];
-    const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
-    if (!(p->final_mode & FFBP_LEVELS_TC2) && ffbp::level_fused_supported(v.C, Lk, v.Dk, Lp, v.Dp)) return 1;
-    return ffbp::level_tc_supported(v.C, Lk, v.Dk) ? 2 : 0;
-}
-
-// The float16 intermediate of the two-pass tensor-core levels: the largest any of them needs.
-static size_t tc_scratch(const ffbp_plan *p)
-{
-    size_t m = 0;
-    for (int l = 0; l < p->nlev; ++l) {
-        if (level_form(p, l) != 2) continue;
-        const DevLevel &v = p->lv[l];
-        m = std::max(m, ffbp::level_tc_scratch_bytes(v.Np, v.C, v.P, v.Ko));
-    }
-    return m;
-}
-
-// Whether any level runs the two-pass kernels, whose intermediate is scaled from the input's largest component
-// (the history's is found by a scan ahead of the first level).
-static bool any_two_pass(const ffbp_plan *p)
-{
-    for (int l = 0; l < p->nlev; ++l)
-        if (level_form(p, l) == 2) return true;
-    return false;
-}
-
 int ffbp_plan_workspace_bytes(const ffbp_plan *p, size_t *bytes)
 {
     if (!p || !bytes) return fail(FFBP_E_ARG, "null argument");
-    *bytes = 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2)) + align256(tc_scratch(p));
+    *bytes = 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2)) + align256(p->scratch);
     return FFBP_OK;
 }
 
@@ -439,7 +501,7 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     };
     mark(0);
     const float2 *in = static_cast<const float2 *>(d_S);
-    if (level_form(p, 0) == 2) {
+    if (two_pass(p->lv[0])) {
         if ((e = ffbp::launch_amax(in, (size_t)p->lv[0].P * p->lv[0].K, amax, s)) != cudaSuccess) return cuda_fail(e, "history scan");
         mark(FFBP_KIND_AMAX << 8);
     }
@@ -457,11 +519,13 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
         L.tc_nt = v.tc.nt; L.tc_sb = v.tc.sb; L.tc_pc = v.tc.copies; L.tc_rp = v.tc.repeat; L.tc_fir = v.tc.fir;
         L.tc_cw = v.tc.consumers;
         const char *why = nullptr;
-        const int form = level_form(p, l);
-        if (form == 1) {
+        if (v.form == LV_ONE_PASS) {
             e = ffbp::launch_level_fused(L, p->d_aborts, s, &why);
             if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC << 8 | l);
-        } else if (form == 2) {
+        } else if (v.form == LV_FP32) {
+            e = ffbp::launch_level(L, s, &why);
+            if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL << 8 | l);
+        } else if (v.form == LV_TWO_PASS_F16) {
             e = ffbp::launch_level_tc_gemm(L, amax + l, scratch, p->d_aborts, s, &why);
             if (!why && e == cudaSuccess) {
                 mark(FFBP_KIND_LEVEL_TC_GEMM << 8 | l);
@@ -469,8 +533,15 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
                 if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC_FIR << 8 | l);
             }
         } else {
-            e = ffbp::launch_level(L, s, &why);
-            if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL << 8 | l);
+            for (int n0 = 0; n0 < v.Np && !why && e == cudaSuccess; n0 += v.nn)
+                for (int j0 = 0; j0 < v.Ko && !why && e == cudaSuccess; j0 += v.nj) {
+                    const int nn = std::min(v.nn, v.Np - n0), nj = std::min(v.nj, v.Ko - j0);
+                    e = ffbp::launch_level_mma(L, amax + l, scratch, false, n0, nn, j0, nj, p->d_aborts, s, &why);
+                    if (why || e != cudaSuccess) break;
+                    mark(FFBP_KIND_LEVEL_TC_GEMM << 8 | l);
+                    e = ffbp::launch_level_fir32(L, amax + l, scratch, n0, nn, j0, nj, s, &why);
+                    if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC_FIR << 8 | l);
+                }
         }
         if (why) return fail(FFBP_E_UNSUPPORTED, "level %d: %s", l, why);
         if (e != cudaSuccess) return cuda_fail(e, "level kernel");
@@ -485,10 +556,11 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     F.test_wait_ns = p->test_kind == FFBP_KIND_FINAL_TC ? p->test_ns : 0u;
     const int fm = p->final_mode & 0xff;
     const char *why = nullptr;
-    e = fm == FFBP_FINAL_FP32 ? ffbp::launch_final_fp32(F, s, &why) : ffbp::launch_final_tc(F, fm, s, &why);
+    const bool cores = fm == FFBP_FINAL_FP32;
+    e = cores ? ffbp::launch_final_fp32(F, s, &why) : ffbp::launch_final_tc(F, fm, s, &why);
     if (why) return fail(FFBP_E_UNSUPPORTED, "final stage: %s", why);
     if (e != cudaSuccess) return cuda_fail(e, "final kernel");
-    mark((fm == FFBP_FINAL_FP32 ? FFBP_KIND_FINAL : FFBP_KIND_FINAL_TC) << 8 | p->nlev);
+    mark((cores ? FFBP_KIND_FINAL : FFBP_KIND_FINAL_TC) << 8 | p->nlev);
     // the abort count back to the host once this call's kernels are done (read by the next call, or below)
     if ((e = cudaMemcpyAsync(p->h_aborts, p->d_aborts, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_fail(e, "status read");
@@ -805,8 +877,9 @@ int ffbp_plan_info(const ffbp_plan *p, int *nlev, int *launches)
     if (nlev) *nlev = p->nlev;
     if (launches) {
         int n = 1;
-        for (int l = 0; l < p->nlev; ++l) n += level_form(p, l) == 2 ? 2 : 1;
-        if (any_two_pass(p) && level_form(p, 0) == 2) n += 1;      // the history scan
+        for (const auto &v : p->lv)
+            n += two_pass(v) ? 2 * ((v.Np + v.nn - 1) / v.nn) * ((v.Ko + v.nj - 1) / v.nj) : 1;
+        if (two_pass(p->lv[0])) n += 1;                            // the history scan
         *launches = n;
     }
     return FFBP_OK;

@@ -51,6 +51,14 @@ cudaError_t launch_level_tc_fir(const LevelLaunch &L, const int *amax_in, const 
                                 cudaStream_t s, const char **why);
 cudaError_t launch_level_fir_tc(const LevelLaunch &L, const int *amax_in, const void *scratch, int *err,
                                 cudaStream_t s, const char **why);
+// The first pass with the window operand read in place (level_mma.cu), whatever the taps and children: parents n0 .. n0 +
+// nn - 1 and output columns j0 .. j0 + nj - 1 into y [nn, C, P, (nj + 3) & ~3], float16 (half) or float32 complex, and
+// the pulse FIR of such a float32 intermediate into its place in L.out.
+bool level_mma_supported(int C, int Lk, int Dk, int Ko);
+cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, bool half, int n0, int nn, int j0,
+                             int nj, int *err, cudaStream_t s, const char **why);
+cudaError_t launch_level_fir32(const LevelLaunch &L, const int *amax_in, const void *y, int n0, int nn, int j0, int nj,
+                               cudaStream_t s, const char **why);
 // The largest |component| of n complex samples into *amax (float bits, atomicMax; start at 0).
 cudaError_t launch_amax(const float2 *x, size_t n, int *amax, cudaStream_t s);
 

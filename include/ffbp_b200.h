@@ -41,30 +41,28 @@ enum {
 
 /* Final-stage arithmetic (ImageFormer's precision=, fastsar/api.py:27-31).                                     */
 enum {
-    FFBP_FINAL_FP32 = 0,    /* float32 on the CUDA cores: the plain path                                        */
+    FFBP_FINAL_FP32 = 0,    /* float32: the plain path (its levels as split float16 products on the tensor cores,  */
+                            /* 22 bits, where the rotation phases are small, else on the CUDA cores)              */
     FFBP_FINAL_TC_F16 = 1,  /* tcgen05 tensor cores, float16 operands, float32 accumulation; ffbp_form scales  */
                             /* the samples by a power of two into float16's range, ffbp_final takes them as    */
                             /* given (each component below 2^14 in magnitude)                                   */
     FFBP_FINAL_TC_BF16X3 = 2, /* tcgen05 tensor cores, operands split x = hi + lo in bfloat16, the hi*hi, hi*lo, */
                               /* lo*hi and lo*lo products accumulated in float32                               */
-    FFBP_LEVELS_TC = 0x100,   /* flag, or-ed into ffbp_plan_desc.final_mode: the levels on the tensor cores     */
-                              /* (per pulse the children's modulated frequency taps times the parent row's      */
-                              /* Hankel windows, three bfloat16 products accumulated in float32), in one pass:  */
+    FFBP_LEVELS_TC = 0x100,   /* flag, or-ed into ffbp_plan_desc.final_mode: the mixed-precision levels on the  */
+                              /* tensor cores (per pulse the children's modulated frequency taps times the      */
+                              /* parent row's windows, three split products accumulated in float32), in one pass: */
                               /* the ramp and the pulse FIR follow each pulse's product on the multiprocessor,  */
                               /* the FIR's running sums in tensor memory. Levels the one-pass kernel does not   */
                               /* cover (more than 8 output pulses per input pulse) take the two-pass form below; */
-                              /* levels of more than 64 children or 96 frequency taps stay on the float32 kernel */
+                              /* levels of more than 64 children or 96 frequency taps keep a float32 intermediate */
     FFBP_LEVELS_TC2 = 0x200   /* flag, with FFBP_LEVELS_TC: every tensor-core level in two passes (the product   */
                               /* and ramp into a float16 intermediate in the workspace, then the pulse FIR in   */
                               /* float32), the form before the one-pass kernel                                    */
 };
 
-/* Launch options of a tensor-core level (level_tc_gemm, and the kernel of its pulse FIR; no counterpart in the
- * reference, whose kernels take fixed shapes). 0 in a field keeps the default. They change the schedule, not the arithmetic: the plane copies
- * and B stages leave every bit as it is; the columns per tile and the row repeat move the points where the output
- * ramp's recurrence is seeded: a rounding-level change (about 1e-7 before the float16 intermediate, whose rounding
- * it can flip by one unit: about 1e-5 relative in all). FFBP_E_UNSUPPORTED (at the form call) for a choice that
- * does not fit.                                                                                                   */
+/* Launch options of a tensor-core level (no counterpart in the reference, whose kernels take fixed shapes). 0 in a
+ * field keeps the default. `fir` chooses the pulse FIR's kernel; the others were those of an earlier first pass: they
+ * are checked as before (FFBP_E_UNSUPPORTED at the form call for a choice that did not fit it) and change nothing.  */
 typedef struct {
     int nt;                 /* output columns per tile: a multiple of 16 (32 with repeated rows), at most 128       */
     int sb;                 /* stages of the B operand ring: 2 to 4                                                 */
@@ -243,9 +241,9 @@ int ffbp_level(const void *d_x, int Np, int P, int K, const void *d_phase, int C
                int Dk, int Ko, double kc, const float *d_tp, int Lp, int plp, int Dp, int Po, const float *d_wp,
                const float *d_wk, void *d_out, int *d_bad, void *stream);
 
-/* The same level on the tensor cores (the arithmetic of FFBP_LEVELS_TC): per pulse the children's modulated
- * frequency taps tk[r] exp(2 pi i sl r) times the Hankel windows of the parent's row, three bfloat16 products
- * accumulated in float32; the ramp exp(2 pi i (c0 + sl (Dk j - plk - kc))); a float16 intermediate in d_scratch
+/* The same level on the tensor cores (the arithmetic of FFBP_LEVELS_TC | FFBP_LEVELS_TC2): per pulse the children's
+ * modulated frequency taps tk[r] exp(2 pi i sl r) times the windows of the parent's row, operands split into float16
+ * hi + lo, three products accumulated in float32; the ramp exp(2 pi i (c0 + sl (Dk j - plk - kc))); a float16 intermediate in d_scratch
  * (ffbp_level_tc_scratch_bytes, 16-byte aligned), scaled by a power of two from the input's largest component;
  * the pulse FIR in float32. C <= 64 and Lk <= 96 (FFBP_E_UNSUPPORTED otherwise). d_status: 3 ints, zeroed by the
  * caller: [0] nonzero when a bounded wait of the kernel ran out, [1] the input's largest |component| (float bits,
