@@ -125,7 +125,8 @@ struct ffbp_plan {
     std::vector<DevLevel> lv;
     float *wp = nullptr, *wk = nullptr, *wf = nullptr;
     double *ux = nullptr, *uy = nullptr, *ucx = nullptr, *ucy = nullptr, *rc = nullptr;
-    float4 *seeds = nullptr;          // the float16 tensor-core final stage's ramp seeds [ntiles, Pf]
+    float4 *seeds = nullptr;          // the tensor-core final stage's ramp seeds [ntiles, Pf], two each in split float16
+    bool final_x2 = false;            // the float32 form's final stage in split float16 on the tensor cores
     int2 *first = nullptr;
     size_t bufA = 0, bufB = 0;
     size_t scratch = 0;               // bytes of the two-pass levels' intermediate
@@ -438,6 +439,14 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
         e = ffbp::launch_final_seeds(p->ux, p->uy, (long)B * d->Pf, p->spx, p->spy, p->a0, p->a1, p->seeds, s);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "final seeds kernel"));
     }
+    // the float32 form: split float16 products on the tensor cores where they cover the shape; with aperture weights,
+    // which nothing bounds to float16's range, the CUDA cores
+    p->final_x2 = (d->final_mode & 0xff) == FFBP_FINAL_FP32 && !p->wf && ffbp::final_tc32_supported(p->T, B, p->Pf, p->Qf);
+    if (p->final_x2) {
+        if ((e = p->alloc(&p->seeds, 2 * (size_t)B * d->Pf)) != cudaSuccess) return cleanup(cuda_fail(e, "allocate final seeds"));
+        e = ffbp::launch_final_seeds2(p->ux, p->uy, (long)B * d->Pf, p->spx, p->spy, p->a0, p->a1, p->seeds, s);
+        if (e != cudaSuccess) return cleanup(cuda_fail(e, "final seeds kernel"));
+    }
     if ((e = p->alloc(&p->d_aborts, 1)) != cudaSuccess || (e = cudaMemsetAsync(p->d_aborts, 0, sizeof(int), s)) != cudaSuccess)
         return cleanup(cuda_fail(e, "allocate the abort count"));
     if ((e = cudaHostAlloc(reinterpret_cast<void **>(&p->h_aborts), sizeof(int), cudaHostAllocDefault)) != cudaSuccess)
@@ -556,7 +565,7 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     F.test_wait_ns = p->test_kind == FFBP_KIND_FINAL_TC ? p->test_ns : 0u;
     const int fm = p->final_mode & 0xff;
     const char *why = nullptr;
-    const bool cores = fm == FFBP_FINAL_FP32;
+    const bool cores = fm == FFBP_FINAL_FP32 && !p->final_x2;
     e = cores ? ffbp::launch_final_fp32(F, s, &why) : ffbp::launch_final_tc(F, fm, s, &why);
     if (why) return fail(FFBP_E_UNSUPPORTED, "final stage: %s", why);
     if (e != cudaSuccess) return cuda_fail(e, "final kernel");

@@ -9,6 +9,13 @@
 // One MMA is M = 128, N = 128, K = 16, and a "unit" is what one accumulator holds:
 //   FFBP_FINAL_TC_BF16X3  one tile, operands split x = hi + lo in bfloat16: A' = [A_hi; A_lo], B' = [B_hi; B_lo], so
 //                         one product gives hi hi, hi lo, lo hi and lo lo of the tile, summed in the epilogue;
+//   the float32 form      one T = 32 or two T = 16 tiles, operands split x = hi + lo in float16 (22 bits; the samples
+//                         scaled by a power of two) the same way. Its error against float64 is that of the CUDA-core
+//                         kernel it replaces (images 1.4e-6 to 2.1e-6 against 1.5e-6 to 8.8e-6): the ramps' seeds
+//                         come from the plan as hi + lo, their steps are computed to float32's rounding by the loader
+//                         warp, and the accumulations are cut into short segments (the tensor core's sums truncate).
+//                         4,096 tiles of 40 x 46: 700 us (CUDA cores 1,714); 107,520 of 44 x 88: 27.6 ms (83.9);
+//                         4,320 of 48 x 97 at T = 16: 894 us (2,057). The producers' conversions bound it.
 //   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal 64 x 64
 //                         blocks of the product are the tiles; or four T = 16 tiles, whose 32 x 32 diagonal blocks
 //                         are, each epilogue warp reading one of them from its own lane quarter. The samples are
@@ -35,6 +42,8 @@
 // touching the barrier again; each issuing thread drains its MMAs (bounded) before the accumulator columns are freed.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -163,7 +172,7 @@ struct TcArgs {
     int B, Pf, Qf, Qfp, S, nunits, nis;
     const double *__restrict__ ux;
     const double *__restrict__ uy;
-    const float4 *__restrict__ seeds;      // float16 form: the ramp seeds per tile and subaperture (or null)
+    const float4 *__restrict__ seeds;      // the ramp seeds per tile and subaperture: float16 one (or null), split float16 two
     double spx, spy, a0, a1, fc2;
     const double *__restrict__ ucx;
     const double *__restrict__ ucy;
@@ -177,6 +186,8 @@ struct TcArgs {
     int *err;
     const int *amax;
     int interleave;                        // the order of the producer warps' items (final_tc_kernel)
+    int nwi;                               // producer items per stage
+    int seg, nsg;                          // final subapertures per accumulation (even unless all), accumulations per unit
     unsigned test_wait_ns;                 // tests only: the issuers' wait on a barrier nothing completes (0: none)
 };
 
@@ -193,14 +204,18 @@ __device__ __forceinline__ float operand_scale(const int *amax)
     return ldexpf(1.f, 13 - ex);
 }
 
-// 8 values -> 16 bytes of operand: float16, or bfloat16 high parts (and the low parts in lo)
-template <bool BF>
+// The operands' arithmetic: float16, or x = hi + lo in bfloat16 (16 bits) or in float16 (22 bits).
+enum Operands { OP_F16 = 0, OP_BF16X2 = 1, OP_F16X2 = 2 };
+
+// 8 values -> 16 bytes of operand: float16, or the high parts (and the low parts in lo)
+template <int OP>
 __device__ __forceinline__ void pack8(const float *v, uint4 &hi, uint4 &lo)
 {
     uint32_t h[4], l[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        if (BF) {
+        l[e] = 0;
+        if (OP == OP_BF16X2) {
             const __nv_bfloat162 x = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
             const float r0 = v[2 * e] - __low2float(x), r1 = v[2 * e + 1] - __high2float(x);
             const __nv_bfloat162 y = __floats2bfloat162_rn(r0, r1);
@@ -209,7 +224,11 @@ __device__ __forceinline__ void pack8(const float *v, uint4 &hi, uint4 &lo)
         } else {
             const __half2 x = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
             h[e] = *reinterpret_cast<const uint32_t *>(&x);
-            l[e] = 0;
+            if (OP == OP_F16X2) {
+                const float2 f = __half22float2(x);
+                const __half2 y = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
+                l[e] = *reinterpret_cast<const uint32_t *>(&y);
+            }
         }
     }
     hi = make_uint4(h[0], h[1], h[2], h[3]);
@@ -222,13 +241,14 @@ __device__ __forceinline__ uint4 flip_sign(uint4 v)
     return make_uint4(v.x ^ sg, v.y ^ sg, v.z ^ sg, v.w ^ sg);
 }
 
-// The tile of slot ts (float16: 128 / (2 TT) tiles per unit, split bfloat16: one) of this block's local unit ul
-// (>= B when none).
-template <bool BF, int TT>
+// Tiles per unit: 128 operand rows hold 2 TT rows per tile, twice that when split.
+template <int OP, int TT> __host__ __device__ constexpr int unit_tiles() { return OP == OP_F16 ? 64 / TT : 32 / TT; }
+
+// The tile of slot ts of this block's local unit ul (>= B when none).
+template <int OP, int TT>
 __device__ __forceinline__ int unit_tile(int ul, int ts)
 {
-    const int u = (int)blockIdx.x + ul * (int)gridDim.x;
-    return BF ? u : (64 / TT) * u + ts;
+    return unit_tiles<OP, TT>() * ((int)blockIdx.x + ul * (int)gridDim.x) + ts;
 }
 
 // The pixels of one T = 32 tile from P0 = D'[0:32, :] and P1 = D'[32:64, :] (rows of 64 + 1 floats in shared
@@ -307,20 +327,21 @@ __device__ __forceinline__ void tile16_pixels(const TcArgs &a, int tile, const f
     }
 }
 
-template <bool BF, bool WEIGHTED, int MAXWI, int TT>
+template <int OP, bool WEIGHTED, int MAXWI, int TT>
 __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
 {
-    constexpr int NTS = BF ? 1 : 64 / TT;                       // tiles per unit
+    constexpr bool BF = OP == OP_BF16X2, X2 = OP == OP_F16X2;
+    constexpr int NTS = unit_tiles<OP, TT>();                   // tiles per unit
     extern __shared__ __align__(1024) unsigned char smem[];
     const int ng = a.Qfp / 8;                                   // core matrices along K per operand
     const uint32_t H = 64u * a.Qfp * 2u;                        // 64 operand rows
-    const uint32_t HS = 2u * TT * a.Qfp * 2u;                   // one tile's operand rows (float16), 2 TT rows
+    const uint32_t HS = 2u * TT * a.Qfp * 2u;                   // one part (hi or lo) of a tile's operand rows, 2 TT rows
     const uint32_t stagebytes = 4u * H;                         // A' (128 rows), B' (128 rows)
     float *sP = reinterpret_cast<float *>(smem + (size_t)a.S * stagebytes);             // [2][32][65]
     // the loader's ring: per slot and tile slot, the subaperture's Qfp samples (zero past Qf), ux, uy and the
-    // three weights (tsb bytes)
+    // three weights (split float16: the seeds of both ramps and the steps of the TT / 2 row pairs of each); tsb bytes
     unsigned char *ring = reinterpret_cast<unsigned char *>(sP + 2 * 32 * 65);
-    const uint32_t tsb = 8u * a.Qfp + 32u, slotbytes = (uint32_t)NTS * tsb;
+    const uint32_t tsb = 8u * a.Qfp + 32u + (X2 ? 8u * TT : 0u), slotbytes = (uint32_t)NTS * tsb;
     uint64_t *bars = reinterpret_cast<uint64_t *>(ring + (size_t)LS * slotbytes);
     uint64_t *full = bars, *empty = bars + a.S, *accf = bars + 2 * a.S, *acce = accf + 2, *drain = acce + 2;
     uint64_t *lfull = drain + 2, *lempty = lfull + LS;
@@ -335,7 +356,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
     if (t == 0) {
         s_abort = 0;
         for (int s = 0; s < a.S; ++s) {
-            mbar_init(&full[s], NPW);
+            mbar_init(&full[s], X2 ? (uint32_t)a.nwi : NPW);
             mbar_init(&empty[s], 1);
         }
         for (int k = 0; k < 2; ++k) {
@@ -344,11 +365,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
             mbar_init(&drain[k], 1);
         }
         for (int k = 0; k < LS; ++k) {
-            mbar_init(&lfull[k], 32);                      // the loader's 32 threads, once their copies have landed
-            mbar_init(&lempty[k], NPW);
+            // the loader's 32 threads, once their copies have landed (split float16: and their steps are written)
+            mbar_init(&lfull[k], X2 ? 64 : 32);
+            mbar_init(&lempty[k], X2 ? (uint32_t)a.nwi : NPW);
         }
         mbar_init(&s_never, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (X2) {                                                   // whole groups past Qf are not written: zero once
+        for (uint32_t i = (uint32_t)t * 16u; i < (uint32_t)a.S * stagebytes; i += NTHREADS * 16u)
+            *reinterpret_cast<uint4 *>(smem + i) = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == NEPI) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -370,24 +397,36 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         const int nts = NTS;
         const int ntot = nul * a.Pf;
         const size_t nbp = (size_t)a.B * a.Pf;
-        const bool fs = !BF && a.seeds;                         // stage the float32 seeds in place of ux, uy
+        const bool fs = OP == OP_F16 && a.seeds;                // stage the float32 seeds in place of ux, uy
         auto prefetch_unit = [&](int ul) {
             if (ul >= nul) return;
             for (int ts = 0; ts < nts; ++ts) {
-                const int tile = unit_tile<BF, TT>(ul, ts);
+                const int tile = unit_tile<OP, TT>(ul, ts);
                 if (tile >= a.B) break;
                 const char *dbeg = reinterpret_cast<const char *>(a.d + (size_t)tile * a.Pf * a.Qf);
                 const int dbytes = a.Pf * a.Qf * (int)sizeof(float2);
                 for (int o = lane * 128; o < dbytes; o += 32 * 128)
                     asm volatile("prefetch.global.L2 [%0];" :: "l"(dbeg + o));
-                const char *src = fs ? reinterpret_cast<const char *>(a.seeds + (size_t)tile * a.Pf)
-                                     : reinterpret_cast<const char *>((lane < 16 ? a.ux : a.uy) + (size_t)tile * a.Pf);
-                const int ub = a.Pf * (fs ? 16 : 8);
+                const char *src = X2   ? reinterpret_cast<const char *>(a.seeds + 2 * (size_t)tile * a.Pf)
+                                  : fs ? reinterpret_cast<const char *>(a.seeds + (size_t)tile * a.Pf)
+                                       : reinterpret_cast<const char *>((lane < 16 ? a.ux : a.uy) + (size_t)tile * a.Pf);
+                const int ub = a.Pf * (X2 ? 32 : fs ? 16 : 8);
                 for (int o = (lane & 15) * 128; o < ub; o += 16 * 128)
                     asm volatile("prefetch.global.L2 [%0];" :: "l"(src + o));
             }
         };
         int ul = 0, p = 0;
+        // split float16: lane l computes the step of row pair r of operand xop of tile slot xts, whose slope it reads
+        // a subaperture ahead
+        const int xts = X2 ? lane / TT : 0, xop = (lane % TT) / (TT / 2), xr = lane % (TT / 2);
+        float2 slope = make_float2(0.f, 0.f);
+        auto fetch_slope = [&](int fu, int fp) {
+            const int tile = fu < nul ? unit_tile<OP, TT>(fu, xts) : a.B;
+            slope = make_float2(0.f, 0.f);
+            if (tile < a.B)
+                slope = *(reinterpret_cast<const float2 *>(a.seeds + 2 * ((size_t)tile * a.Pf + fp) + xop) + 1);
+        };
+        if (X2) fetch_slope(0, 0);
         for (int it = 0; it < ntot; ++it) {
             const int ls = it % LS;
             if (it >= LS && !mbar_wait<PRODUCER_HINT_NS>(&lempty[ls], (uint32_t)((it / LS - 1) & 1), &s_abort, a.err))
@@ -395,7 +434,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
             if (p == 0) prefetch_unit(ul + 1);
             const uint32_t sl = smem_u32(ring) + (uint32_t)ls * slotbytes;
             for (int ts = 0; ts < nts; ++ts) {
-                const int tile = unit_tile<BF, TT>(ul, ts);
+                const int tile = unit_tile<OP, TT>(ul, ts);
                 const bool tv = tile < a.B;
                 const size_t bp = tv ? (size_t)tile * a.Pf + p : 0;
                 const float2 *src = a.d + bp * a.Qf;
@@ -405,7 +444,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     cp_async(dst + 8u * q, v ? (const void *)(src + q) : (const void *)a.d, 8, v);
                 }
                 const uint32_t gd = dst + 8u * a.Qfp;
-                if (fs) {
+                if (X2) {
+                    if (lane < 2) cp_async(gd + 16u * lane, (const void *)(a.seeds + 2 * bp + lane), 16, tv);
+                } else if (fs) {
                     if (lane == 0) cp_async(gd, (const void *)(a.seeds + bp), 16, tv);
                 } else if (lane < 2) cp_async(gd + 8u * lane, (const void *)((lane ? a.uy : a.ux) + bp), 8, tv);
                 else if (WEIGHTED && lane < 5)
@@ -413,8 +454,128 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&lfull[ls])) : "memory");
             if (++p == a.Pf) { p = 0; ++ul; }
+            if (X2) {
+                const float m = (float)(2 * xr - (TT - 1));
+                float c = m * slope.x;                          // exact; the low part then moves it by a rounding
+                c = (c - rintf(c)) + m * slope.y;
+                float sn, cs;
+                sincospif(-2.f * c, &sn, &cs);
+                *reinterpret_cast<float2 *>(ring + (size_t)ls * slotbytes + (uint32_t)xts * tsb + 8u * a.Qfp + 32u +
+                                            8u * (uint32_t)(xop * (TT / 2) + xr)) = make_float2(cs, sn);
+                mbar_arrive(&lfull[ls]);
+                fetch_slope(ul, p);
+            }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (X2 && warp >= PW0) {
+        // ------------------------------------------------------------------ producers, split float16
+        // Items, lanes and rows as below. Here the items (twice the conversions and stores) alternate A, the heavier,
+        // and B, and are dealt to the warps in turn from a start that moves by one more than their count per stage: every
+        // warp gets as many of each and runs ahead over the ring (a stage is full once its nwi items have arrived; a
+        // fixed set of items per warp and stage was 1.4 times slower at 40 x 46).
+        const int pw = warp - PW0;
+        constexpr int GPI = 64 / TT;
+        const int ngr = (a.Qf + 7) / 8, hg = (ngr + GPI - 1) / GPI, ntot = nul * a.Pf;
+        const int r = lane % (TT / 2), sub = lane / (TT / 2);
+        uint32_t roff[4];
+        {
+            const int rows[4] = {r, r + TT, TT - 1 - r, 2 * TT - 1 - r};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) roff[k] = (uint32_t)(((rows[k] >> 3) * ng) * 128 + (rows[k] & 7) * 16);
+        }
+        const float dscale = operand_scale(a.amax), m = (float)(2 * r - (TT - 1));
+        const int rs = a.S / nis, turn = (a.nwi + 1) % NPW;
+        int ps0 = 0, ps1 = 0, p = 0, first = pw;
+        uint32_t pp0 = 0, pp1 = 0;
+        for (int it = 0; it < ntot; ++it) {
+            const int ls = it % LS, kq = nis == 2 ? (p & 1) : 0, stg = kq + nis * (kq ? ps1 : ps0);
+            if (first < a.nwi &&
+                !(mbar_wait<PRODUCER_HINT_NS>(&lfull[ls], (uint32_t)((it / LS) & 1), &s_abort, a.err) &&
+                  mbar_wait<PRODUCER_HINT_NS>(&empty[stg], (kq ? pp1 : pp0) ^ 1u, &s_abort, a.err)))
+                break;
+            for (int item = first; item < a.nwi; item += NPW) {
+                const int q = item >> 1, ts = NTS == 1 ? 0 : q / hg, g = GPI * (NTS == 1 ? q : q - ts * hg) + sub;
+                const bool isA = (item & 1) == 0;
+                if (g < ngr) {
+                    const unsigned char *tsp = ring + (size_t)ls * slotbytes + (uint32_t)ts * tsb;
+                    // the ramp at sample 8 g: -(m Y + 8 g m V) cycles from the plan's seeds, whose high parts times m
+                    // and 8 g m are exact
+                    const float4 sd = *reinterpret_cast<const float4 *>(tsp + 8 * a.Qfp + (isA ? 0 : 16));
+                    const float n8 = m * (8.f * (float)g);
+                    float c0 = m * sd.x, c1 = n8 * sd.z;
+                    c0 -= rintf(c0);
+                    c1 -= rintf(c1);
+                    float2 wv = cis_cycles(-((c0 + c1) + fmaf(m, sd.y, n8 * sd.w)));
+                    const float2 st = *reinterpret_cast<const float2 *>(tsp + 8 * a.Qfp + 32 + 8 * ((isA ? 0 : TT / 2) + r));
+                    unsigned char *ob = smem + (size_t)stg * stagebytes + (isA ? 0u : 2u * H) + (uint32_t)ts * (2u * HS) + (uint32_t)g * 128u;
+                    uint4 h, l;
+                    if (isA) {
+                        wv.x *= dscale;
+                        wv.y *= dscale;
+                        const float4 *dq = reinterpret_cast<const float4 *>(tsp + 64 * g);
+                        float r1[8], i1[8], r2[8], i2[8];
+#pragma unroll
+                        for (int e2 = 0; e2 < 4; ++e2) {
+                            const float4 dd = dq[e2];
+#pragma unroll
+                            for (int hh = 0; hh < 2; ++hh) {
+                                const int e = 2 * e2 + hh;
+                                const float dr = hh ? dd.z : dd.x, di = hh ? dd.w : dd.y;
+                                const float pr = dr * wv.x, pi = di * wv.x;
+                                r1[e] = fmaf(-di, wv.y, pr); i1[e] = fmaf(dr, wv.y, pi);   // d x
+                                r2[e] = fmaf(di, wv.y, pr); i2[e] = fmaf(-dr, wv.y, pi);   // d conj(x)
+                                wv = cmul(wv, st);
+                            }
+                        }
+                        pack8<OP>(r1, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[0]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[0]) = l;
+                        pack8<OP>(i1, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[1]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[1]) = l;
+                        pack8<OP>(r2, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[2]) = l;
+                        pack8<OP>(i2, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[3]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[3]) = l;
+                    } else {
+                        float r1[8], i1[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            r1[e] = wv.x;
+                            i1[e] = wv.y;
+                            wv = cmul(wv, st);
+                        }
+                        pack8<OP>(r1, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[0]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[0]) = l;
+                        *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[2]) = l;
+                        pack8<OP>(i1, h, l);
+                        *reinterpret_cast<uint4 *>(ob + roff[1]) = h;
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[1]) = l;
+                        *reinterpret_cast<uint4 *>(ob + roff[3]) = flip_sign(h);
+                        *reinterpret_cast<uint4 *>(ob + HS + roff[3]) = flip_sign(l);
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&full[stg]);
+                    mbar_arrive(&lempty[ls]);
+                }
+            }
+            first -= turn;
+            if (first < 0) first += NPW;
+            if (kq) {
+                if (++ps1 == rs) { ps1 = 0; pp1 ^= 1u; }
+            } else if (++ps0 == rs) {
+                ps0 = 0;
+                pp0 ^= 1u;
+            }
+            if (++p == a.Pf) p = 0;
+        }
     } else if (warp >= PW0) {
         // ------------------------------------------------------------------ producers
         // Warp items: (tile slot ts, operand A or B, pair of 8-sample groups gp). Lane l of the warp takes pixel
@@ -535,24 +696,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 }
                 uint4 h, l;
                 const bool mirror = !isA && !WEIGHTED;
-                pack8<BF>(r1, h, l);
+                pack8<OP>(r1, h, l);
                 *reinterpret_cast<uint4 *>(ob + roff[0]) = h;
                 if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[0]) = l;
                 if (mirror) {
                     *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[2]) = l;
                 }
-                pack8<BF>(i1, h, l);
+                pack8<OP>(i1, h, l);
                 *reinterpret_cast<uint4 *>(ob + roff[1]) = h;
                 if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[1]) = l;
                 if (mirror) {
                     *reinterpret_cast<uint4 *>(ob + roff[3]) = flip_sign(h);
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[3]) = flip_sign(l);
                 } else {
-                    pack8<BF>(r2, h, l);
+                    pack8<OP>(r2, h, l);
                     *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[2]) = l;
-                    pack8<BF>(i2, h, l);
+                    pack8<OP>(i2, h, l);
                     *reinterpret_cast<uint4 *>(ob + roff[3]) = h;
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[3]) = l;
                 }
@@ -588,14 +749,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
             // tests of the failure report: a wait that runs out before any MMA, as a stuck pipeline's would
             const bool stuck = a.test_wait_ns &&
                                !mbar_wait<ISSUER_HINT_NS>(&s_never, 0, &s_abort, a.err, a.test_wait_ns);
-            for (int ul = stuck ? nul : 0; ul < nul; ++ul) {
-                const int ab = ul & 1;
-                if (!mbar_wait<ISSUER_HINT_NS>(&acce[ab], (uint32_t)(((ul >> 1) & 1) ^ 1), &s_abort, a.err)) break;
+            // an accumulation j (segment sg of unit ul) goes into this issuer's accumulator j mod 2
+            int sg = 0;
+            for (int j = 0, nj = stuck ? 0 : nul * a.nsg; j < nj; ++j) {
+                const int ab = j & 1;
+                if (!mbar_wait<ISSUER_HINT_NS>(&acce[ab], (uint32_t)(((j >> 1) & 1) ^ 1), &s_abort, a.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t dt = tmem + (uint32_t)((k * 2 + ab) * 128);
                 bool ok = true;
                 uint32_t accum = 0;
-                for (int p = k; p < a.Pf; p += nis) {
+                const int p1 = min(a.Pf, (sg + 1) * a.seg);
+                for (int p = sg * a.seg + k; p < p1; p += nis) {
                     const int stg = k + nis * slot;
                     if (!mbar_wait<ISSUER_HINT_NS>(&full[stg], par, &s_abort, a.err)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -609,6 +773,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 }
                 if (!ok) break;
                 mma_commit(&accf[ab]);
+                if (++sg == a.nsg) sg = 0;
             }
         }
         __syncwarp();
@@ -619,13 +784,76 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         // after a failed wait a warp keeps stepping through the units (and the epilogue's named barriers, which all
         // four warps must reach) without waiting, reading or writing
         bool live = true;
+        int j = 0;                                              // accumulations read
         for (int ul = 0; ul < nul; ++ul) {
+            const uint32_t lanes = (uint32_t)(32 * warp) << 16;
+            float *mine = (warp & 1) ? P1 : P0;                 // accumulator rows 32..63 (mod 64) are the Ai rows
+            if (OP == OP_F16X2) {
+                // The tensor core's float32 sums truncate: a chain of n of them loses about n 3e-8 of the result. So a
+                // unit is accumulated in segments, added here in float32 with rounding. This thread's accumulator row,
+                // hi and lo columns summed:
+                constexpr int NV = TT == 32 ? 64 : 32;
+                float v[NV];
+#pragma unroll
+                for (int i = 0; i < NV; ++i) v[i] = 0.f;
+                const int c0 = TT == 32 ? 0 : 64 * (warp >> 1);
+                for (int sg = 0; sg < a.nsg; ++sg, ++j) {
+                    const int ab = j & 1, na = min(nis, a.Pf - sg * a.seg);   // issuers with a stage in the segment
+                    if (live) live = mbar_wait<EPILOGUE_HINT_NS>(&accf[ab], (uint32_t)((j >> 1) & 1), &s_abort, a.err);
+                    live = __all_sync(0xffffffffu, live);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (!live) continue;
+                    for (int k = 0; k < na; ++k) {
+                        const uint32_t base = tmem + lanes + (uint32_t)((k * 2 + ab) * 128 + c0);
+#pragma unroll
+                        for (int c = 0; c < NV; c += 16) {
+                            uint32_t q0[16], q1[16];
+                            tmem_ld16(base + (uint32_t)c, q0);
+                            tmem_ld16(base + (uint32_t)(NV + c), q1);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) v[c + i] += __uint_as_float(q0[i]) + __uint_as_float(q1[i]);
+                        }
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acce[ab]);
+                }
+                if (TT == 32) {
+                    // warps 0, 1: the hi rows; then warps 2, 3 add the lo rows
+                    if (live && warp < 2) {
+#pragma unroll
+                        for (int i = 0; i < NV; ++i) mine[lane * 65 + i] = v[i];
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (live && warp >= 2) {
+#pragma unroll
+                        for (int i = 0; i < NV; ++i) mine[lane * 65 + i] += v[i];
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (live) tile_pixels(a, unit_tile<OP, TT>(ul, 0), P0, P1, t, oscale);
+                } else {
+                    // tile slot ts = warp / 2: the hi rows (Re, Im) in the even warp's lanes, the lo rows in the odd one's
+                    const int ts = warp >> 1;
+                    float *part = sP + ts * (32 * 33) + lane * 33;
+                    if (live && (warp & 1)) {
+#pragma unroll
+                        for (int i = 0; i < NV; ++i) part[i] = v[i];
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (live && !(warp & 1)) {
+#pragma unroll
+                        for (int i = 0; i < NV; ++i) v[i] += part[i];
+                        tile16_pixels(a, unit_tile<OP, TT>(ul, ts), v, v + 16, lane, oscale);
+                    }
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                continue;
+            }
             const int ab = ul & 1;
             if (live) live = mbar_wait<EPILOGUE_HINT_NS>(&accf[ab], (uint32_t)((ul >> 1) & 1), &s_abort, a.err);
             live = __all_sync(0xffffffffu, live);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t lanes = (uint32_t)(32 * warp) << 16;
-            float *mine = (warp & 1) ? P1 : P0;                 // accumulator rows 32..63 (mod 64) are the Ai rows
             // the sum over the issuers' accumulators of columns [c0, c0 + 16), plus [c0 + c1, c0 + c1 + 16) if c1
             auto gather = [&](int c0, int c1, float *v) {
                 uint32_t q0[16], q1[16];
@@ -640,7 +868,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(q0[j]) + (c1 ? __uint_as_float(q1[j]) : 0.f);
                 }
             };
-            if (BF) {
+            if (OP == OP_BF16X2) {
                 // warps 0, 1: hi rows (hi hi + hi lo); then warps 2, 3 add the lo rows (lo hi + lo lo)
                 float v[16];
                 if (live && warp < 2) {
@@ -667,7 +895,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     if (lane == 0) mbar_arrive(&acce[ab]);
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (live) tile_pixels(a, unit_tile<BF, TT>(ul, 0), P0, P1, t, oscale);
+                if (live) tile_pixels(a, unit_tile<OP, TT>(ul, 0), P0, P1, t, oscale);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             } else if (TT == 16) {
                 // tile slot ts = warp: accumulator rows [32 ts, 32 ts + 32) (this warp's lane quarter) at columns
@@ -679,7 +907,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acce[ab]);
-                    tile16_pixels(a, unit_tile<BF, TT>(ul, warp), v0, v1, lane, oscale);
+                    tile16_pixels(a, unit_tile<OP, TT>(ul, warp), v0, v1, lane, oscale);
                 }
             } else {
                 // tile slot ts: accumulator rows and columns [64 ts, 64 ts + 64), read by warps 2 ts and 2 ts + 1
@@ -697,7 +925,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                         if (lane == 0) mbar_arrive(&acce[ab]);
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    const int tile = unit_tile<BF, TT>(ul, ts);
+                    const int tile = unit_tile<OP, TT>(ul, ts);
                     if (live && tile < a.B) tile_pixels(a, tile, P0, P1, t, oscale);
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
@@ -733,7 +961,34 @@ __global__ void final_seeds_kernel(const double *__restrict__ ux, const double *
     }
 }
 
+// The split float16 form's seeds of one ramp: Y = frac(u sp a0 / 2) and V = u sp a1 / 2 as hi + lo, Y's high part of 18
+// bits (times a row's m, |m| < 32, exact) and V's of 11 (times 8 g m, below 2^13, exact).
+__device__ __forceinline__ float4 split_seed(double u, double sp, double a0, double a1)
+{
+    const double y = 0.5 * u * sp * a0, V = 0.5 * u * sp * a1, Y = y - floor(y);
+    const float yh = (float)(rint(Y * 262144.0) / 262144.0), vf = (float)V, t = vf * 8193.f, vh = t - (t - vf);
+    return make_float4(yh, (float)(Y - (double)yh), vh, (float)(V - (double)vh));
+}
+
+__global__ void final_seeds2_kernel(const double *__restrict__ ux, const double *__restrict__ uy, long n, double spx,
+                                    double spy, double a0, double a1, float4 *__restrict__ out)
+{
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        out[2 * i] = split_seed(ux[i], spx, a0, a1);
+        out[2 * i + 1] = split_seed(uy[i], spy, a0, a1);
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_final_seeds2(const double *ux, const double *uy, long n, double spx, double spy, double a0,
+                                double a1, float4 *out, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    const long nb = (n + 255) / 256;
+    final_seeds2_kernel<<<(int)(nb < 4096 ? nb : 4096), 256, 0, s>>>(ux, uy, n, spx, spy, a0, a1, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_final_seeds(const double *ux, const double *uy, long n, double spx, double spy, double a0,
                                double a1, float4 *out, cudaStream_t s)
@@ -744,68 +999,103 @@ cudaError_t launch_final_seeds(const double *ux, const double *uy, long n, doubl
     return cudaGetLastError();
 }
 
+namespace {
+
+struct TcShape { int nts, nwi, maxwi, S; size_t smem; };
+
+// The unit and the ring of a final stage's shape (op: Operands); false with *why for shapes the kernel does not cover.
+bool tc_shape(int op, int T, int Pf, int Qf, size_t maxsmem, TcShape *o, const char **why)
+{
+    const bool split = op != OP_F16;
+    if (T != 32 && (T != 16 || op == OP_BF16X2)) {
+        *why = "the tensor-core final stage takes T = 32 (split bfloat16 or float16) or T = 16 (float16)";
+        return false;
+    }
+    // warp items per stage: (tile slots) x (A, B) x (pairs of 8-sample groups) over the NPW producer warps
+    const int Qfp = (Qf + 15) & ~15, gpi = 64 / T, hg = ((op == OP_F16X2 ? (Qf + 7) / 8 : Qfp / 8) + gpi - 1) / gpi;
+    o->nts = (split ? 32 : 64) / T;
+    o->nwi = o->nts * 2 * hg;
+    o->maxwi = (o->nwi + NPW - 1) / NPW;
+    if (o->maxwi > 4) { *why = "more than 256 frequency samples per final tile"; return false; }
+    const int nis = Pf >= NISS ? NISS : 1;
+    const size_t stage = (size_t)4 * 64 * Qfp * 2;
+    const size_t slotbytes = (size_t)o->nts * (8 * Qfp + 32 + (op == OP_F16X2 ? 8 * T : 0));
+    const size_t fixed = (size_t)2 * 32 * 65 * 4 + (size_t)LS * slotbytes + (size_t)(2 * 4 + 6 + 2 * LS) * 8;
+    const size_t avail = maxsmem - 1024;                        // static shared memory and slack
+    // stages: a multiple of the issuers (each owns S / nis of them)
+    int S = 4;
+    while (S > 2 && ((size_t)S * stage + fixed > avail || S % nis)) --S;
+    if ((size_t)S * stage + fixed > avail) {
+        *why = "a final subaperture's operands do not fit shared memory (Qf too large for the tensor-core stage)";
+        return false;
+    }
+    o->S = S;
+    o->smem = (size_t)S * stage + fixed;
+    return true;
+}
+
+size_t max_smem()
+{
+    int dev = 0, v = 227 * 1024;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return (size_t)v;
+}
+
+}  // namespace
+
+bool final_tc32_supported(int T, int B, int Pf, int Qf)
+{
+    const char *why = nullptr;
+    TcShape o;
+    return (long long)B * Pf < (1LL << 31) && tc_shape(OP_F16X2, T, Pf, Qf, max_smem(), &o, &why);
+}
+
 cudaError_t launch_final_tc(const FinalLaunch &F, int mode, cudaStream_t s, const char **why)
 {
     *why = nullptr;
-    const bool bf = mode == 2;
-    if (F.T != 32 && (F.T != 16 || bf)) {
-        *why = "the tensor-core final stage takes T = 32 (split bfloat16 or float16) or T = 16 (float16)";
-        return cudaErrorNotSupported;
-    }
+    const int op = mode == 0 ? OP_F16X2 : (mode == 2 ? OP_BF16X2 : OP_F16);
+    TcShape o;
+    if (!tc_shape(op, F.T, F.Pf, F.Qf, max_smem(), &o, why)) return cudaErrorNotSupported;
     if (F.B <= 0) return cudaSuccess;
     if ((long long)F.B * F.Pf >= (1LL << 31)) { *why = "more than 2^31 final tile subapertures"; return cudaErrorNotSupported; }
-    const int nts = bf ? 1 : 64 / F.T;                          // tiles per unit
     TcArgs a;
     a.d = F.d; a.B = F.B; a.Pf = F.Pf; a.Qf = F.Qf; a.Qfp = (F.Qf + 15) & ~15;
-    a.nunits = (F.B + nts - 1) / nts;
+    a.nunits = (F.B + o.nts - 1) / o.nts;
     a.nis = F.Pf >= NISS ? NISS : 1;
+    a.nwi = o.nwi; a.S = o.S;
+    // when every producer warp gets the same even number of items they are interleaved (as many A items, the heavier,
+    // as B items on each warp: 3 % faster at 47 x 91 in float16; 1 % slower at 38 x 71, whose count is uneven)
+    a.interleave = o.nwi % (2 * NPW) == 0 ? 1 : 0;
+    // split float16: accumulations of about 24 steps (an even count of subapertures for two issuers)
+    const int per = std::max(1, 24 / (a.Qfp / 16));
+    a.seg = op == OP_F16X2 ? std::min(F.Pf, a.nis * per) : F.Pf;
+    a.nsg = (F.Pf + a.seg - 1) / a.seg;
     a.ux = F.ux; a.uy = F.uy; a.seeds = F.seeds; a.spx = F.spx; a.spy = F.spy; a.a0 = F.a0; a.a1 = F.a1; a.fc2 = F.fc2;
     a.ucx = F.ucx; a.ucy = F.ucy; a.rc = F.rc; a.w = F.w; a.tiles = F.tiles; a.img = F.img; a.first = F.first;
     a.nx = F.nx; a.ny = F.ny; a.ox = F.ox; a.oy = F.oy; a.scale = F.scale; a.err = F.err; a.amax = F.amax;
     a.test_wait_ns = F.test_wait_ns;
-    int dev = 0, nsm = 148, maxsmem = 227 * 1024;
+    int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    // warp items per stage: (tile slots) x (A, B) x (pairs of 8-sample groups) over the NPW producer warps; when
-    // every warp gets the same even number of items they are interleaved (as many A items, the heavier, as B
-    // items on each warp: 3 % faster at 47 x 91 in float16; 1 % slower at 38 x 71, whose count is uneven)
-    const int ng = a.Qfp / 8, gpi = 64 / F.T, hg = (ng + gpi - 1) / gpi;
-    const int nwi = nts * 2 * hg;
-    a.interleave = nwi % (2 * NPW) == 0 ? 1 : 0;
-    const int maxwi = (nwi + NPW - 1) / NPW;
-    if (maxwi > 4) { *why = "more than 256 frequency samples per final tile"; return cudaErrorNotSupported; }
-    const int mw = maxwi <= 1 ? 1 : (maxwi <= 2 ? 2 : 4);
-    const size_t stage = (size_t)4 * 64 * a.Qfp * 2;
-    const size_t slotbytes = (size_t)nts * (8 * a.Qfp + 32);
-    const size_t fixed = (size_t)2 * 32 * 65 * 4 + (size_t)LS * slotbytes + (size_t)(2 * 4 + 6 + 2 * LS) * 8;
-    const size_t avail = (size_t)maxsmem - 1024;                // static shared memory and slack
-    // stages: a multiple of the issuers (each owns S / nis of them)
-    int S = 4;
-    while (S > 2 && ((size_t)S * stage + fixed > avail || S % a.nis)) --S;
-    if ((size_t)S * stage + fixed > avail) {
-        *why = "a final subaperture's operands do not fit shared memory (Qf too large for the tensor-core stage)";
-        return cudaErrorNotSupported;
-    }
-    a.S = S;
-    const size_t smem = (size_t)S * stage + fixed;
     const int grid = a.nunits < nsm ? a.nunits : nsm;
     auto run = [&](auto kern) -> cudaError_t {
-        cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o.smem);
         if (r != cudaSuccess) return r;
-        kern<<<grid, NTHREADS, smem, s>>>(a);
+        kern<<<grid, NTHREADS, o.smem, s>>>(a);
         return cudaGetLastError();
     };
+    if (op == OP_F16X2) {
+        // weighted tiles: a pulse's weight has no bound that float16's range could be held to
+        if (a.w || !a.seeds) { *why = "the split float16 final stage takes the plan's seeds and no aperture weights"; return cudaErrorNotSupported; }
+        return F.T == 16 ? run(final_tc_kernel<OP_F16X2, false, 1, 16>) : run(final_tc_kernel<OP_F16X2, false, 1, 32>);
+    }
 #define FFBP_TC_RUN(MW)                                                                                       \
-    (bf ? (a.w ? run(final_tc_kernel<true, true, MW, 32>) : run(final_tc_kernel<true, false, MW, 32>))        \
-        : F.T == 16 ? (a.w ? run(final_tc_kernel<false, true, MW, 16>) : run(final_tc_kernel<false, false, MW, 16>)) \
-                    : (a.w ? run(final_tc_kernel<false, true, MW, 32>) : run(final_tc_kernel<false, false, MW, 32>)))
-    cudaError_t e;
-    if (mw == 1) e = FFBP_TC_RUN(1);
-    else if (mw == 2) e = FFBP_TC_RUN(2);
-    else e = FFBP_TC_RUN(4);
+    (op == OP_BF16X2 ? (a.w ? run(final_tc_kernel<OP_BF16X2, true, MW, 32>) : run(final_tc_kernel<OP_BF16X2, false, MW, 32>)) \
+     : F.T == 16     ? (a.w ? run(final_tc_kernel<OP_F16, true, MW, 16>) : run(final_tc_kernel<OP_F16, false, MW, 16>))   \
+                     : (a.w ? run(final_tc_kernel<OP_F16, true, MW, 32>) : run(final_tc_kernel<OP_F16, false, MW, 32>)))
+    return o.maxwi <= 1 ? FFBP_TC_RUN(1) : o.maxwi <= 2 ? FFBP_TC_RUN(2) : FFBP_TC_RUN(4);
 #undef FFBP_TC_RUN
-    return e;
 }
 
 }  // namespace ffbp

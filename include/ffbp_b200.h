@@ -41,8 +41,10 @@ enum {
 
 /* Final-stage arithmetic (ImageFormer's precision=, fastsar/api.py:27-31).                                     */
 enum {
-    FFBP_FINAL_FP32 = 0,    /* float32: the plain path (its levels as split float16 products on the tensor cores,  */
-                            /* 22 bits, where the rotation phases are small, else on the CUDA cores)              */
+    FFBP_FINAL_FP32 = 0,    /* float32: the plain path. Where they cover the shape, its final stage (without       */
+                            /* aperture weights) and its levels of small rotation phases run as split float16      */
+                            /* products (22 bits, float32 sums) on the tensor cores, else on the CUDA cores;       */
+                            /* ffbp_final takes the CUDA cores                                                     */
     FFBP_FINAL_TC_F16 = 1,  /* tcgen05 tensor cores, float16 operands, float32 accumulation; ffbp_form scales  */
                             /* the samples by a power of two into float16's range, ffbp_final takes them as    */
                             /* given (each component below 2^14 in magnitude)                                   */
