@@ -158,8 +158,15 @@ cudaError_t launch_fir(FirArgs f, cudaStream_t s)
 {
     constexpr int APP = (AP + 3) & ~3;
     const long nb = ((long)f.rows * ((f.nj + 1) / 2) + 127) / 128;
+    // segments of output pulses: the count whose waves of blocks (about 8 a multiprocessor) times the pulses a thread
+    // sweeps (its outputs' and the AP - 1 of its halo) are fewest (the 512-pixel spotlight's first level: 1 segment 60
+    // us, 7 segments 16)
     int nseg = 1;
-    while (nb * nseg < 148L * 16 && f.Po / (nseg * 2) >= 8 * AP) nseg *= 2;
+    double best = 1e30;
+    for (int k = 1; k <= 64 && k <= f.Po; ++k) {
+        const double w = (double)nb * k / (148.0 * 8), cost = (w < 8 ? std::ceil(w) : w) * ((f.Po + k - 1) / k + AP - 1);
+        if (cost < best) { best = cost; nseg = k; }
+    }
     f.SEG = (f.Po + nseg - 1) / nseg;
     f.nseg = (f.Po + f.SEG - 1) / f.SEG;
     if (nb > 0x7fffffffL || f.nseg > 65535) return cudaErrorInvalidValue;
