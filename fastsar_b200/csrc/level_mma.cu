@@ -21,8 +21,11 @@
 // the products' error is 2^-22, below that of the float32 sums; with a full row of 8 taps a step is 16 long (8 real, 8
 // imaginary parts).
 //
+// The first level's window lies in shared memory (K floats) where it fits: read through L1, which the operands leave
+// little of, its latency bound the sample warps (2,048 x 2,048 float32: 886 -> 524 us).
+//
 // Measured (B200, first passes of the levels in us, against the kernel that copied the windows into Hankel rows): the
-// 12,288 x 8,832 spotlight's mixed form 5,350 / 4,830 / 6,200 (7,570 / 7,210 / 12,890), the 1,499 x 701 patch at T = 16
+// 12,288 x 8,832 spotlight's mixed form 4,610 / 4,830 / 6,200 (7,570 / 7,210 / 12,890), the 1,499 x 701 patch at T = 16
 // 265 / 348 / 439 (840 / 850 / 895), the 512-pixel spotlight 25 / 23 / 38 (221 / 88 / 96). The sine, cosine and stores of
 // the read-out and, with few children, the latency of a pulse's chain of roles bound it; the MMAs take a quarter to a half.
 //
@@ -51,6 +54,7 @@ constexpr int M_NTHR = 512;
 constexpr int M_PB = 8;                      // pulses per batch of child phases
 constexpr int M_PHB = 3;                     // ring of phase batches
 constexpr int M_ND = 4;                      // most accumulator buffers
+constexpr int M_NBAR = 2 * 4 + 2 * 4 + 2 * M_ND + 2 * M_PHB + 2;   // barriers
 constexpr uint64_t M_WAIT_NS = 2000000000ull;
 constexpr float M_TAP_SCALE = 8.f;           // the taps' power of two; the samples' is y_scale / M_TAP_SCALE
 
@@ -71,6 +75,7 @@ struct MmaArgs {
     int TM, ntile, TG, ntg;           // column steps per tile, tiles of TM S columns, tiles per unit, units per row
     int ROWS, W;                      // rows of a plane, staged samples of a tile
     int NT, ZS, XR, nd;               // buffers: taps, planes, staged samples, accumulators
+    int wtab;                         // the window's samples in shared memory (K floats)
     int TW;                           // tap warps that build a unit's taps together (4, or 1 a unit each with NT = 4)
     long nunits;
     float kc;
@@ -138,22 +143,39 @@ __device__ __forceinline__ bool elect_one()
     return p != 0;
 }
 
+// GC consecutive columns of this thread's lane (not waited for)
+template <int GC>
+__device__ __forceinline__ void tmem_ldc(uint32_t addr, float *v)
+{
+    if constexpr (GC == 8) {
+        tmem_ld8(addr, v);
+    } else {
+        uint32_t r[4];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+    }
+}
+
 // Dynamic shared memory: taps [NT][hi, lo][ks][2][N][16 B], planes [ZS][S][G][re hi, im hi, re lo, im lo][ROWS][16 B],
 // staged samples [XR][W], the phase batches [PHB][PB][Ch] (float4: c0, sl, the phasor of Dk samples; float2: of one),
 // the taps' values [ks][8], the barriers.
 __host__ __device__ constexpr size_t mma_tap_bytes(int Ch, int ks) { return (size_t)2 * ks * 2 * (2 * Ch) * 16; }
 __host__ __device__ constexpr size_t mma_plane_bytes(int S, int G, int rows) { return (size_t)S * G * 4 * rows * 16; }
-__host__ __device__ constexpr size_t mma_raw_bytes(int W) { return ((size_t)W * 8 + 15) & ~(size_t)15; }
-__host__ __device__ constexpr size_t mma_smem(int S, int G, int rows, int W, int Ch, int ks, int NT, int ZS, int XR)
+// (16 bytes on: the pulse's window weight)
+__host__ __device__ constexpr size_t mma_raw_bytes(int W) { return (((size_t)W * 8 + 15) & ~(size_t)15) + 16; }
+__host__ __device__ constexpr size_t mma_smem(int S, int G, int rows, int W, int Ch, int ks, int NT, int ZS, int XR,
+                                              size_t wtab)
 {
     // a product always reads 128 rows from its first: with shorter planes the last one's overrun (at most 96 rows, whose
     // accumulator rows nobody reads) ends inside what follows the planes
     const size_t after = XR * mma_raw_bytes(W) + (size_t)M_PHB * M_PB * Ch * 24 + (size_t)ks * 32 +
-                         (size_t)(2 * 4 + 2 * 4 + 2 * M_ND + 2 * M_PHB + 2) * 8;
+                         (size_t)M_NBAR * 8 + wtab;
     return NT * mma_tap_bytes(Ch, ks) + ZS * mma_plane_bytes(S, G, rows) + (after > 96 * 16 ? after : 96 * 16);
 }
 
-template <int S, bool HALF, bool WIN>
+template <int S, bool HALF, bool WIN, int GC>
 __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -168,6 +190,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
     float2 *sS = reinterpret_cast<float2 *>(sP + (size_t)M_PHB * M_PB * a.Ch); // [PHB][PB][Ch]: a sample's phasor
     float *sH = reinterpret_cast<float *>(sS + (size_t)M_PHB * M_PB * a.Ch);   // [ks][8]
     uint64_t *bars = reinterpret_cast<uint64_t *>(sH + (size_t)a.ks * 8);
+    float *sW = reinterpret_cast<float *>(bars + M_NBAR);                       // [K] the window's samples (wtab)
     uint64_t *tfull = bars, *tempty = tfull + 4, *zfull = tempty + 4, *zempty = zfull + 4, *dfull = zempty + 4,
              *dempty = dfull + M_ND, *pfull = dempty + M_ND, *pempty = pfull + M_PHB, *drain = pempty + M_PHB,
              *never = drain + 1;
@@ -194,6 +217,8 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
         const int r = Dks * ia + 8 * g + e;
         sH[i] = (8 * g + e < Dks && r < a.Lk) ? (a.tk ? a.tk[r] : 1.f) * M_TAP_SCALE : 0.f;
     }
+    if (WIN && a.wtab)
+        for (int i = t; i < a.K; i += M_NTHR) sW[i] = a.wk ? a.wk[i] : 1.f;
     if (warp == M_MW) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_u32(&s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -291,6 +316,9 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
                                  :: "r"(dst + 8u * i), "l"(v ? row + k : a.x), "r"(v ? 8 : 0) : "memory");
                 }
+                if (WIN && xt == 0)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;"
+                                 :: "r"(dst + rawbytes - 16u), "l"(a.wp + ld.p) : "memory");
                 if (++lslot == a.XR) lslot = 0;
                 if (++ltl == min(a.ntile, (ld.tg + 1) * a.TG)) {
                     ld.next(a);
@@ -313,7 +341,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                 unsigned char *zb = sZ + (size_t)zs * zbytes;
                 const int rows = rows_of(tl), items = rows * a.G * S;
                 const int kb = a.Dk * (a.j0 + tl * a.TM * S) - a.plk;
-                const float wpp = WIN ? a.wp[un.p] : 1.f;
+                const float wpp = WIN ? *reinterpret_cast<const float *>(sR + (size_t)slot * rawbytes + rawbytes - 16) : 1.f;
                 uint32_t worst = 0;
                 int m = xt, gr = 0;
                 while (m >= rows) { m -= rows; ++gr; }
@@ -328,7 +356,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                             v = raw[o + e];
                             if (WIN) {
                                 const int k = min(max(kb + o + e, 0), a.K - 1);
-                                const float w = wpp * __ldg(&a.wk[k]);   // the reference's float32 window product
+                                const float w = wpp * (a.wtab ? sW[k] : a.wk ? __ldg(&a.wk[k]) : 1.f);   // the reference's float32 window product
                                 v.x *= w;
                                 v.y *= w;
                             }
@@ -487,8 +515,8 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
         }
     } else {
         // ------------------------------------------------------------------ consumers
-        // Warp w: accumulator lanes 32 (w % 4) .. + 31 (an output column step each), the groups of 8 children of
-        // parity w / 4. A thread's S columns S j' .. S j' + S - 1 are adjacent.
+        // Warp w: accumulator lanes 32 (w % 4) .. + 31 (an output column step each), the groups of GC children of
+        // parity w / 4 (4 where there are few). A thread's S columns S j' .. S j' + S - 1 are adjacent.
         constexpr int SP = S < 2 ? 1 : 2;                       // columns read together
         const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
         Unit un;
@@ -522,22 +550,22 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                 const uint32_t base = tmem + lanes + (uint32_t)(d * S) * N;
                 const size_t yo = (((size_t)un.n * a.C + un.cg * a.Ch) * a.P + un.p) * a.Kop + j;
                 if (any) {
-                    for (int cb = 8 * (warp >> 2); cb < nc; cb += 16) {
+                    for (int cb = GC * (warp >> 2); cb < nc; cb += 2 * GC) {
 #pragma unroll
                         for (int r0 = 0; r0 < S; r0 += SP) {
-                            float re[SP][8], im[SP][8];
+                            float re[SP][GC], im[SP][GC];
 #pragma unroll
                             for (int r = 0; r < SP; ++r) {
-                                tmem_ld8(base + (uint32_t)((r0 + r) * N + cb), re[r]);
-                                tmem_ld8(base + (uint32_t)((r0 + r) * N + a.Ch + cb), im[r]);
+                                tmem_ldc<GC>(base + (uint32_t)((r0 + r) * N + cb), re[r]);
+                                tmem_ldc<GC>(base + (uint32_t)((r0 + r) * N + a.Ch + cb), im[r]);
                             }
                             tmem_wait_ld();
-                            // the ramps of the 8 children side by side (no branch between them: the chain phase ->
+                            // the ramps of the children side by side (no branch between them: the chain phase ->
                             // sine and cosine -> product is long), children past nc computed and not stored
                             const float u = uf + (float)(r0 * a.Dk);
-                            float2 e[8];
+                            float2 e[GC];
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) {
+                            for (int c = 0; c < GC; ++c) {
                                 const float2 q = *reinterpret_cast<const float2 *>(&pr[cb + c]);
                                 // in float32 with the product's rounding error carried along (hundreds of cycles leave
                                 // few bits for the fraction), which float16 does not need
@@ -551,7 +579,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
 #pragma unroll
                             for (int r = 0; r < SP; ++r)
 #pragma unroll
-                                for (int c = 0; c < 8; ++c) {
+                                for (int c = 0; c < GC; ++c) {
                                     const float2 o = cmul(make_float2(re[r][c], im[r][c]), e[c]);
                                     re[r][c] = o.x;
                                     im[r][c] = o.y;
@@ -562,7 +590,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                                 if (HALF) {
                                     __half2 *yp = static_cast<__half2 *>(a.y) + at;
 #pragma unroll
-                                    for (int c = 0; c < 8; ++c) {
+                                    for (int c = 0; c < GC; ++c) {
                                         const __half2 v0 = __floats2half2_rn(re[0][c], im[0][c]), v1 = __floats2half2_rn(re[SP - 1][c], im[SP - 1][c]);
                                         if (cb + c < nc) {
                                             if (SP == 1) *yp = v0;
@@ -574,7 +602,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
                                 } else {
                                     float2 *yp = static_cast<float2 *>(a.y) + at;
 #pragma unroll
-                                    for (int c = 0; c < 8; ++c) {
+                                    for (int c = 0; c < GC; ++c) {
                                         if (cb + c < nc) {
                                             if (SP == 1) *yp = make_float2(re[0][c], im[0][c]);
                                             else *reinterpret_cast<float4 *>(yp) = make_float4(re[0][c], im[0][c], re[SP - 1][c], im[SP - 1][c]);
@@ -620,7 +648,7 @@ struct MmaShape { int S, TM, G, A, ks, Ch, ROWS, W, NT, ZS, XR; size_t smem; };
 // The shape of a level's product: the residues S and the column steps per tile TM (fewer than 128 only where long
 // filters at large decimations leave no room) that need the fewest MMA cycles for the row's tiles, and the most children
 // per group whose operands fit with two tap buffers (one where that doubles the group).
-bool mma_shape(int C, int Lk, int Dk, int nj, MmaShape *out)
+bool mma_shape(int C, int Lk, int Dk, int nj, size_t wtab, MmaShape *out)
 {
     long best = 0;
     for (int TM = 128; TM >= 32 && !best; TM /= 2)
@@ -643,14 +671,14 @@ bool mma_shape(int C, int Lk, int Dk, int nj, MmaShape *out)
             for (const auto &o : opt) {
                 int ch = cmax;
                 if (o[0] == 4 && s.ks * std::min(cmax, (C + 7) & ~7) > TW1_ITEMS) continue;
-                while (ch >= 8 && mma_smem(S, s.G, s.ROWS, s.W, ch, s.ks, o[0], o[1], o[2]) > MMA_SMEM_MAX) ch -= 8;
+                while (ch >= 8 && mma_smem(S, s.G, s.ROWS, s.W, ch, s.ks, o[0], o[1], o[2], wtab) > MMA_SMEM_MAX) ch -= 8;
                 if (ch < 8) continue;
                 const int g = (C + ch - 1) / ch;
                 if (g * 2 > groups) continue;                // fewer buffers only for half the groups
                 groups = g;
                 s.NT = o[0]; s.ZS = o[1]; s.XR = o[2];
                 s.Ch = (((C + g - 1) / g) + 7) & ~7;
-                s.smem = mma_smem(S, s.G, s.ROWS, s.W, s.Ch, s.ks, s.NT, s.ZS, s.XR);
+                s.smem = mma_smem(S, s.G, s.ROWS, s.W, s.Ch, s.ks, s.NT, s.ZS, s.XR, wtab);
             }
             if (!s.Ch) continue;
             const int ntile = (nj + TM * S - 1) / (TM * S);
@@ -669,7 +697,7 @@ bool mma_shape(int C, int Lk, int Dk, int nj, MmaShape *out)
 bool level_mma_supported(int C, int Lk, int Dk, int Ko)
 {
     MmaShape s;
-    return C >= 1 && Dk >= 1 && Lk >= 1 && Lk <= 512 && mma_shape(C, Lk, Dk, Ko, &s);
+    return C >= 1 && Dk >= 1 && Lk >= 1 && Lk <= 512 && mma_shape(C, Lk, Dk, Ko, 0, &s);
 }
 
 cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, bool half, int n0, int nn, int j0,
@@ -678,13 +706,17 @@ cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, 
     *why = nullptr;
     const int Lk = L.Dk > 1 ? L.Lk : 1, plk = L.Dk > 1 ? L.plk : 0;
     MmaShape m;
-    if (!mma_shape(L.C, Lk, L.Dk, nj, &m)) { *why = "the level's operands do not fit shared memory"; return cudaErrorNotSupported; }
+    // the first level's window over the samples in shared memory, where that costs no children per group
+    const size_t wtab = L.wp ? ((size_t)L.K * 4 + 15) & ~(size_t)15 : 0;
+    MmaShape m0;
+    const bool tab = wtab && mma_shape(L.C, Lk, L.Dk, nj, wtab, &m) && mma_shape(L.C, Lk, L.Dk, nj, 0, &m0) && m.Ch == m0.Ch;
+    if (!tab && !mma_shape(L.C, Lk, L.Dk, nj, 0, &m)) { *why = "the level's operands do not fit shared memory"; return cudaErrorNotSupported; }
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     MmaArgs a;
     a.x = L.x; a.ph = L.phase; a.tk = L.Dk > 1 ? L.tk : nullptr; a.wp = L.wp; a.wk = L.wk; a.bad = L.bad;
-    a.amax_in = amax_in; a.y = y; a.err = err; a.n0 = n0; a.C = L.C; a.P = L.P; a.K = L.K; a.Dk = L.Dk; a.Lk = Lk;
+    a.amax_in = amax_in; a.y = y; a.err = err; a.wtab = tab; a.n0 = n0; a.C = L.C; a.P = L.P; a.K = L.K; a.Dk = L.Dk; a.Lk = Lk;
     a.plk = plk; a.j0 = j0; a.nj = nj; a.Kop = (nj + 3) & ~3; a.G = m.G; a.A = m.A; a.ks = m.ks; a.Ch = m.Ch;
     a.ncg = (L.C + m.Ch - 1) / m.Ch; a.TM = m.TM; a.ntile = (nj + m.TM * m.S - 1) / (m.TM * m.S);
     a.ROWS = m.ROWS; a.W = m.W; a.NT = m.NT; a.ZS = m.ZS; a.XR = m.XR; a.TW = m.NT == 4 ? 1 : M_NTW;
@@ -705,10 +737,12 @@ cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, 
         return cudaGetLastError();
     };
     const bool win = L.wp != nullptr;
-#define FFBP_MMA_RUN(SV)                                                                                    \
-    (half ? (win ? run(level_mma_kernel<SV, true, true>) : run(level_mma_kernel<SV, true, false>))           \
-          : (win ? run(level_mma_kernel<SV, false, true>) : run(level_mma_kernel<SV, false, false>)))
+#define FFBP_MMA_RUN2(SV, GV)                                                                               \
+    (half ? (win ? run(level_mma_kernel<SV, true, true, GV>) : run(level_mma_kernel<SV, true, false, GV>))   \
+          : (win ? run(level_mma_kernel<SV, false, true, GV>) : run(level_mma_kernel<SV, false, false, GV>)))
+#define FFBP_MMA_RUN(SV) (m.Ch <= 16 ? FFBP_MMA_RUN2(SV, 4) : FFBP_MMA_RUN2(SV, 8))
     return m.S == 4 ? FFBP_MMA_RUN(4) : m.S == 2 ? FFBP_MMA_RUN(2) : FFBP_MMA_RUN(1);
+#undef FFBP_MMA_RUN2
 #undef FFBP_MMA_RUN
 }
 
