@@ -1114,6 +1114,17 @@ int ffbp_final(const void *d_d, int B, int Pf, int Qf, int T, const double *d_ux
     return FFBP_OK;
 }
 
+int ffbp_bp_pad(const void *d_S, int c128, int n, int K, const float *d_wp, const float *d_wk, int nfft, void *d_pad,
+                void *stream)
+{
+    if (!d_S || !d_pad || (!d_wp != !d_wk)) return fail(FFBP_E_ARG, "ffbp_bp_pad: null buffer");
+    if (n < 0 || K < 1 || nfft < K || (nfft > 1 && (nfft & 1))) return fail(FFBP_E_ARG, "ffbp_bp_pad: %d samples into rows of %d", K, nfft);
+    cudaError_t e = ffbp::launch_bp_pad(d_S, c128, n, K, d_wp, d_wk, nfft, static_cast<double2 *>(d_pad),
+                                        static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "ffbp_bp_pad");
+    return FFBP_OK;
+}
+
 int ffbp_bp_points_f64(const void *d_prof, int P, int nfft, const double *d_tx, const double *d_rcv,
                        const double *d_ref, const double *d_pts, long N, double inv_dr, double kcyc, void *d_out,
                        void *stream)

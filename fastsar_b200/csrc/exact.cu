@@ -15,16 +15,20 @@ namespace ffbp {
 
 namespace {
 
-__global__ void bp_points_f64_kernel(const double2 *__restrict__ prof, int P, int nfft, const double *__restrict__ tx,
-                                     const double *__restrict__ rcv, const double *__restrict__ ref,
-                                     const double *__restrict__ pts, long N, double inv_dr, double kcyc,
-                                     double2 *__restrict__ out)
+// LPP lanes share a point, each taking every LPP-th pulse, and add their sums by shuffles: with a thread per point a few
+// thousand points leave most of the device idle behind one thread's chain of dependent reads (20,000 points: 157 blocks). The launch takes the fewest lanes that fill the device.
+template <int LPP>
+__global__ void __launch_bounds__(128) bp_points_f64_kernel(const double2 *__restrict__ prof, int P, int nfft,
+                                                            const double *__restrict__ tx, const double *__restrict__ rcv,
+                                                            const double *__restrict__ ref, const double *__restrict__ pts,
+                                                            long N, double inv_dr, double kcyc, double2 *__restrict__ out)
 {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    const double x = pts[3 * n], y = pts[3 * n + 1], z = pts[3 * n + 2];
+    const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x, n = gid / LPP;
+    const int l = (int)(gid % LPP);
+    const bool in = n < N;
+    const double x = in ? pts[3 * n] : 0.0, y = in ? pts[3 * n + 1] : 0.0, z = in ? pts[3 * n + 2] : 0.0;
     double ar = 0.0, ai = 0.0;
-    for (int p = 0; p < P; ++p) {
+    for (int p = l; in && p < P; p += LPP) {
         const double ax = x - tx[3 * p], ay = y - tx[3 * p + 1], az = z - tx[3 * p + 2];
         double dR = sqrt(ax * ax + ay * ay + az * az);
         if (rcv) {
@@ -47,7 +51,33 @@ __global__ void bp_points_f64_kernel(const double2 *__restrict__ prof, int P, in
         ar += vr * c - vi * s;
         ai += vr * s + vi * c;
     }
-    out[n] = make_double2(out[n].x + ar, out[n].y + ai);
+#pragma unroll
+    for (int o = LPP / 2; o > 0; o >>= 1) {
+        ar += __shfl_xor_sync(0xffffffffu, ar, o);
+        ai += __shfl_xor_sync(0xffffffffu, ai, o);
+    }
+    if (in && l == 0) out[n] = make_double2(out[n].x + ar, out[n].y + ai);
+}
+
+// The rows of S (complex64, or complex128) windowed (the float32 product wp[p] wk[k], then the sample times it in
+// float32), times (-1)^i at place i of the zero-padded row, sample K / 2 at place 0: the unscaled inverse transform of
+// the row is then the profile with zero delay at nfft / 2 (nfft even: the sign is the half-length shift, exactly).
+template <class T>
+__global__ void bp_pad_kernel(const T *__restrict__ S, long n, int K, const float *__restrict__ wp,
+                              const float *__restrict__ wk, int nfft, double2 *__restrict__ pad)
+{
+    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n * K; q += (long)gridDim.x * blockDim.x) {
+        const long p = q / K;
+        const int k = (int)(q - p * K), h = K / 2, i = k >= h ? k - h : nfft - h + k;
+        const T v = S[q];
+        double2 o = make_double2(v.x, v.y);
+        if (wp) {
+            const float w = __fmul_rn(wp[p], wk[k]);
+            o = make_double2(__fmul_rn((float)v.x, w), __fmul_rn((float)v.y, w));
+        }
+        const double g = (i & 1) ? -1.0 : 1.0;
+        pad[p * nfft + i] = make_double2(o.x * g, o.y * g);
+    }
 }
 
 constexpr int SIM_NT = 256;
@@ -136,7 +166,29 @@ cudaError_t launch_bp_points_f64(const double2 *prof, int P, int nfft, const dou
 {
     if (N <= 0 || P <= 0) return cudaSuccess;
     const int nt = 128;
-    bp_points_f64_kernel<<<(unsigned)((N + nt - 1) / nt), nt, 0, s>>>(prof, P, nfft, tx, rcv, ref, pts, N, inv_dr, kcyc, out);
+    int lpp = 1;
+    while (lpp < 32 && N * lpp < 148L * 2048 && P >= 16 * lpp) lpp *= 2;
+    const unsigned nb = (unsigned)((N * lpp + nt - 1) / nt);
+    auto run = [&](auto kern) { kern<<<nb, nt, 0, s>>>(prof, P, nfft, tx, rcv, ref, pts, N, inv_dr, kcyc, out); };
+    switch (lpp) {
+        case 1: run(bp_points_f64_kernel<1>); break;
+        case 2: run(bp_points_f64_kernel<2>); break;
+        case 4: run(bp_points_f64_kernel<4>); break;
+        case 8: run(bp_points_f64_kernel<8>); break;
+        case 16: run(bp_points_f64_kernel<16>); break;
+        default: run(bp_points_f64_kernel<32>); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bp_pad(const void *S, int c128, long n, int K, const float *wp, const float *wk, int nfft,
+                          double2 *pad, cudaStream_t s)
+{
+    if (n <= 0 || K <= 0) return cudaSuccess;
+    const long nb = (n * K + 255) / 256;
+    const unsigned g = (unsigned)(nb < 148 * 16 ? nb : 148 * 16);
+    if (c128) bp_pad_kernel<<<g, 256, 0, s>>>(static_cast<const double2 *>(S), n, K, wp, wk, nfft, pad);
+    else bp_pad_kernel<<<g, 256, 0, s>>>(static_cast<const float2 *>(S), n, K, wp, wk, nfft, pad);
     return cudaGetLastError();
 }
 

@@ -110,6 +110,8 @@ cudaError_t launch_final_seeds2(const double *ux, const double *uy, long n, doub
 cudaError_t launch_bp_points_f64(const double2 *prof, int P, int nfft, const double *tx, const double *rcv,
                                  const double *ref, const double *pts, long N, double inv_dr, double kcyc, double2 *out,
                                  cudaStream_t s);
+cudaError_t launch_bp_pad(const void *S, int c128, long n, int K, const float *wp, const float *wk, int nfft,
+                          double2 *pad, cudaStream_t s);
 cudaError_t launch_simulate(const double *ant, int P, int K, double fmin, double df, const double *pos,
                             const double2 *amp, int N, float2 *S, cudaStream_t s);
 

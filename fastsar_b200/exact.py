@@ -18,18 +18,6 @@ def plane_points(nx, ny, spx, spy, e1=(1.0, 0.0, 0.0), e2=(0.0, 1.0, 0.0), heigh
     return p
 
 
-def _range_compress_device(S, nfft):
-    """S [p, K] complex (torch, device) -> [p, nfft] complex128 range profiles (zero delay at nfft // 2, the carrier of
-    sample K // 2 removed, the unnormalised inverse transform; fastsar/bp.py:55-63) by cuFFT."""
-    import torch
-    P, K = S.shape
-    h = K // 2
-    pad = torch.zeros((P, nfft), dtype=torch.complex128, device=S.device)
-    pad[:, :K - h] = S[:, h:]
-    pad[:, nfft - h:] = S[:, :h]
-    return torch.fft.fftshift(torch.fft.ifft(pad, dim=1), dim=1) * nfft
-
-
 def backproject_device(S, ant, fmin, df, points, *, rcv=None, ref=None, upsample=8, window=True, chunk=256):
     """Exact backprojection at points [..., 3] on the GPU in float64 throughout (profiles, geometry, interpolation,
     phase, accumulation) -> complex128 torch tensor [...] on the device. S: [P, K] complex, numpy or torch."""
@@ -43,11 +31,13 @@ def backproject_device(S, ant, fmin, df, points, *, rcv=None, ref=None, upsample
     tx = np.ascontiguousarray(ant, np.float64)
     if ref is None:
         ref = np.linalg.norm(tx, axis=1) if rcv is None else 0.5 * (np.linalg.norm(tx, axis=1) + np.linalg.norm(rcv, axis=1))
+    # complex64 rows, windowed in float32; wider ones stay in float64 without a window
+    narrow = window or St.dtype in (torch.complex64, torch.float32, torch.float16, torch.bfloat16)
+    St = St.to(torch.complex64 if narrow else torch.complex128).contiguous()
+    wp = wk = None
     if window:
         from .api import _window
-        wp, wk = _window(P, K)
-        w = torch.from_numpy((wp[:, None] * wk[None, :]).astype(np.float32)).to(dev)
-        St = St.to(torch.complex64) * w
+        wp, wk = (torch.from_numpy(v).to(dev) for v in _window(P, K))
     pts_np = np.asarray(points, np.float64)
     shape = pts_np.shape[:-1]
     pts = torch.from_numpy(np.ascontiguousarray(pts_np.reshape(-1, 3))).to(dev)
@@ -59,11 +49,16 @@ def backproject_device(S, ant, fmin, df, points, *, rcv=None, ref=None, upsample
     rcd = None if rcv is None else torch.from_numpy(np.ascontiguousarray(rcv, np.float64)).to(dev)
     refd = torch.from_numpy(np.ascontiguousarray(ref, np.float64)).to(dev)
     s = torch.cuda.current_stream(dev).cuda_stream
+    # per chunk: the windowed, zero-padded rows in one pass, their unscaled inverse transform (cuFFT), the sums
+    pad = torch.zeros((min(chunk, P), nfft), dtype=torch.complex128, device=dev)
     for p0 in range(0, P, chunk):
-        p1 = min(P, p0 + chunk)
-        prof = _range_compress_device(St[p0:p1], nfft).contiguous()
-        _lib.check(L.ffbp_bp_points_f64(prof.data_ptr(), p1 - p0, nfft, txd[p0:p1].data_ptr(),
-                                        None if rcd is None else rcd[p0:p1].data_ptr(), refd[p0:p1].data_ptr(),
+        n = min(P, p0 + chunk) - p0
+        _lib.check(L.ffbp_bp_pad(St[p0].data_ptr(), int(St.dtype == torch.complex128), n, K,
+                                 None if wp is None else wp[p0:].data_ptr(), _lib.tptr(wk), nfft, pad.data_ptr(), s),
+                   'ffbp_bp_pad')
+        prof = torch.fft.ifft(pad[:n], dim=1, norm='forward')
+        _lib.check(L.ffbp_bp_points_f64(prof.data_ptr(), n, nfft, txd[p0:].data_ptr(),
+                                        None if rcd is None else rcd[p0:].data_ptr(), refd[p0:].data_ptr(),
                                         pts.data_ptr(), pts.shape[0], inv_dr, kcyc, out.data_ptr(), s),
                    'ffbp_bp_points_f64')
         del prof

@@ -349,6 +349,13 @@ int ffbp_final(const void *d_d, int B, int Pf, int Qf, int T, const double *d_ux
 
 /* ---- exact backprojection and synthesis (the oracle family, on the device) ----------------------------------- */
 
+/* The rows of that transform (no counterpart in the reference's API): n pulses of d_S [n, K] complex64 (c128 0) or
+ * complex128 (c128 1) into d_pad [n, nfft] complex128, whose other places are zero: with d_wp [n], d_wk [K] each sample
+ * times wp[p] wk[k] in float32; sample K / 2 at place 0, and the sign (-1)^i at place i, so that the unscaled inverse
+ * transform of a row is its profile with zero delay at nfft / 2. nfft even, at least K.                            */
+int ffbp_bp_pad(const void *d_S, int c128, int n, int K, const float *d_wp, const float *d_wk, int nfft, void *d_pad,
+                void *stream);
+
 /* Exact backprojection at N points in float64 (fastsar/bp.py:99-137 bp_points, with float64 profiles): for each point
  * and pulse p, dR = |x - tx[p]| (+ |x - rcv[p]| halved, when d_rcv is not NULL) - ref[p], the profile read at bin
  * dR inv_dr + nfft/2 by linear interpolation, circularly, times exp(2 pi i kcyc dR), accumulated into d_out.
