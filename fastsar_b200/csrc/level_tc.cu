@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(128) level_fir(const FirArgs a)
         for (int s = 0; s < AP; ++s) acc[h][s] = make_float2(0.f, 0.f);
     float vmax = 0.f;
     // input pulses p_start .. p_stop - 1 in chunks of U, the next chunk's loads in flight while one is filtered
-    constexpr int U = 8;
+    constexpr int U = F32 ? 4 : 8;                        // float32: fewer registers, more warps (605 -> 533 us at 30 children
+                                                          // x 448 parents of the 12,288 x 8,832 spotlight's third level)
     const int p_start = a.Dp * i_s - a.plp, p_stop = a.Dp * g_end - a.plp;
     auto ld = [&](int pp) -> PT { return (pp >= 0 && pp < a.P) ? __ldg(yr + (size_t)pp * ypitch) : PT{}; };
     PT cur[U], nxt[U];
