@@ -411,7 +411,7 @@ def main():
     line = dict(
         metric=METRIC, value=value, unit='GBP/s', n_gpus=world, steps=args.steps, warmup=args.warmup,
         ms_per_step=ms, higher_is_better=True, scaling='weak', vs_baseline=None,
-        dtype='mixed: bf16x3 and f16 tensor products, f16 intermediate, f32 accumulation',
+        dtype='mixed: f16x2 (22-bit) and f16 tensor products, f16 intermediate, f32 accumulation',
         data=f'synthetic: {w["n_scatterers"]} seeded scatterers simulated on the GPU in float64, noise -40 dB',
         config=bench_config(args, w, world),
         form_plan=dict(T=chosen.T, taps=[(l['kind_k'], l['kind_p']) for l in plan['levels']],
@@ -550,7 +550,7 @@ def run_patches(args):
         metric='aggregate giga-backprojections/s of 48 uneven patches from 6 collections, one CUDA graph',
         value=bp / (ms_batch * 1e-3) / 1e9, unit='GBP/s', n_gpus=1, steps=args.steps, warmup=args.warmup,
         ms_per_step=ms_batch, higher_is_better=True, scaling='weak', vs_baseline=None,
-        dtype='per patch: the chosen form (bf16x3 / f16 tensor products, f32 accumulation) or float32',
+        dtype='per patch: the chosen form (f16x2 / f16 tensor products, f32 accumulation) or float32',
         data='synthetic: 6 seeded spotlight collections simulated on the GPU in float64, noise -40 dB',
         config=dict(workload='patches_48: 48 patches, sides 256-4096 px (log-uniform, within the unambiguous '
                              'extents), from 6 collections of 2048-16384 pulses x 2048-8192 samples',
@@ -665,7 +665,7 @@ def run_stack(args):
         metric='aggregate giga-backprojections/s of an 8-pass repeat-pass stack, one CUDA graph',
         value=bp / (ms_batch * 1e-3) / 1e9, unit='GBP/s', n_gpus=1, steps=args.steps, warmup=args.warmup,
         ms_per_step=ms_batch, higher_is_better=True, scaling='weak', vs_baseline=None,
-        dtype='mixed: bf16x3 and f16 tensor products, f16 intermediate, f32 accumulation',
+        dtype='mixed: f16x2 (22-bit) and f16 tensor products, f16 intermediate, f32 accumulation',
         data=f'synthetic: one seeded scene of {len(amp)} scatterers, 8 passes simulated on the GPU in float64, '
              'noise -40 dB',
         config=dict(workload='stack_8: 8 passes, 32768 pulses x 4096 samples, Ku 16 GHz, 800 MHz, 6 deg, 50 km, '

@@ -14,9 +14,9 @@ restated); the formation runs in the CUDA library (fastsar_b200/libffbp_b200.so)
 Backends: 'auto' and 'cuda' run on the GPU. There is no CPU, JAX or TPU path in this package; asking for one raises
 ValueError, as the reference does for a backend its machine lacks.
 
-Precision: 'float32' (default): float32 arithmetic everywhere, the final stage on the CUDA cores or, where built,
-as three bfloat16 products on the tensor cores (the reference's float32 CUDA default, fastsar/ffbp_cuda.py:949-953);
-FASTSAR_FINAL=fp32 keeps the CUDA cores. 'float16': the final stage's operands in float16 on the tensor cores with
+Precision: 'float32' (default): float32 arithmetic, or split float16 products (22 bits) accumulated in float32 on the
+tensor cores: the final stage (without an aperture weight) and the levels of small rotation phases. FASTSAR_FINAL=tc3
+takes the final stage in split bfloat16 (the reference's float32 CUDA default, fastsar/ffbp_cuda.py:949-953). 'float16': the final stage's operands in float16 on the tensor cores with
 float32 accumulation (T = 16 or 32).
 """
 import ctypes
@@ -100,8 +100,8 @@ def _check_grid(nx, ny, spx, spy, e1, e2):
 
 
 def _final_mode(precision):
-    """The formation mode of a precision: 'float32' the float32 kernels (FASTSAR_FINAL=tc3 puts the final stage on
-    the tensor cores in split bfloat16); 'float16' the levels and the final stage on the tensor cores, the levels in
+    """The formation mode of a precision: 'float32' the float32 form (FASTSAR_FINAL=tc3 puts its final stage
+    in split bfloat16); 'float16' the levels and the final stage on the tensor cores, the levels in
     two passes through a float16 intermediate (FASTSAR_LEVELS=tc1: in one pass; fp32: on the float32 kernel)."""
     if precision == 'float16':
         lv = os.environ.get('FASTSAR_LEVELS', 'tc').strip().lower() or 'tc'
@@ -318,8 +318,8 @@ class ImageFormer:
     weight of pulses in the final stage (final_weights); ref [P] is the one-way range each pulse is referenced to
     when it is not |ant|. One former must not be called from two threads at once.
 
-    precision='float32' runs the float32 kernels with the reference's filters (70 dB stop band); 'float16' is the
-    mixed-precision form: the levels and the final stage on the tensor cores (split bfloat16 products, a float16
+    precision='float32' runs in float32 with the reference's filters (70 dB stop band); 'float16' is the
+    mixed-precision form: the levels and the final stage on the tensor cores (split float16 products, a float16
     intermediate, float16 final operands, float32 accumulation) with 80 dB filters, whose smaller error leaves room
     for the reduced-precision arithmetic. Unlike the reference's precision='float16' (float16 storage on its own
     plan), this changes the plan's filters: 80 dB instead of 70 dB (unless atten is given); T is chosen as for
@@ -328,10 +328,9 @@ class ImageFormer:
     taps (an extension too): 'kaiser' (default, the reference's Kaiser-sinc decimators), 'learned' (the packaged
     learned decimation taps, fastsar_b200.learned: 8-output-sample filters where the network covers a level's
     decimation and pass fraction, Kaiser-sinc ones elsewhere) or a LearnedTaps instance. tune_levels (an extension):
-    with precision='float16', time the tensor-core levels' launch options (columns per tile, operand stages, plane
-    copies, row repeat, consumer warps, the pulse FIR on the tensor or the CUDA cores) per level shape on the GPU when the former is
-    built (fastsar_b200.tune.tune_levels; cached
-    per shape in the process); the choice changes the image at the rounding level only (about 1e-5 relative: a
+    with precision='float16', time the tensor-core levels' launch options (the pulse FIR on the tensor or the CUDA
+    cores) per level shape on the GPU when the former is built (fastsar_b200.tune.tune_levels; cached per shape in the
+    process); the choice changes the image at the rounding level only (about 1e-5 relative: a
     float16 rounding of the intermediate flipped here and there)."""
 
     def __init__(self, ant, fmin, df, K, nx, ny, spx, spy, e1=(1.0, 0.0, 0.0), e2=(0.0, 1.0, 0.0), *, backend='auto',

@@ -134,22 +134,10 @@ def level_signature(lv, Np):
             int(lv['Dp']), int(Lp))
 
 
-def _level_candidates(C, Lk):
-    """Launch option sets of a tensor-core level in the order a coordinate search visits them: the pulse FIR's kernel
-    (CUDA or tensor cores), plane copies, consumer warps (8, 4 or 12; 16 less them copy Hankel rows), then columns per
-    tile (the multiples of 8 x consumer warps / 4 that the launcher takes), then the row repeat off, then the B
-    stages."""
-    Lkp = ((max(Lk, 1) + 15) // 16) * 16
-    rep_ok = Lkp > 32 and C <= 32
-    return dict(fir=[1, 2], copies=[2, 4], consumers=[8, 4, 12],
-                nt={8: list(range(32, 129, 32)), 4: list(range(16, 129, 16)), 12: list(range(24, 129, 24))},
-                nt16=list(range(16, 129, 16)), repeat_off=rep_ok, sb=[2, 3, 4])
-
-
 def tune_level(lv, Np, reps=3, max_parents=1024, seed=0):
-    """The fastest launch options (ffbp_tc_opts as a dict) of one tensor-core level's first pass, timed with CUDA
-    events on random samples and child phases of the level's shapes and its own filters (at most max_parents
-    parents: the timing is linear in them beyond a few waves), by a coordinate search from the defaults. Results are
+    """The fastest launch options (ffbp_tc_opts as a dict; the one that changes the schedule is the pulse FIR's kernel)
+    of one tensor-core level, timed with CUDA events on random samples and child phases of the level's shapes and its
+    own filters (at most max_parents parents: the timing is linear in them beyond a few waves). Results are
     cached by level_signature. -> (opts, table [(opts, ms or reason)]); opts None when the level is not a
     tensor-core level."""
     import ctypes
@@ -214,26 +202,10 @@ def tune_level(lv, Np, reps=3, max_parents=1024, seed=0):
         if best_ms is None:
             _LEVEL_CACHE[key] = None
             return None, table
-        cand = _level_candidates(C, Lk)
-
-        def consider(o):
-            nonlocal best, best_ms
-            ms = timed(o)
+        for k in (1, 2):                              # the pulse FIR on the CUDA cores, on the tensor cores
+            ms = timed(dict(fir=k))
             if ms is not None and ms < best_ms:
-                best, best_ms = dict(o), ms
-        for k in cand['fir']:
-            consider(dict(best, fir=k))
-        for c in cand['copies']:
-            consider(dict(best, copies=c))
-        for c in cand['consumers']:
-            consider(dict(best, consumers=c))
-        for nt in cand['nt'][best.get('consumers', 8)]:
-            consider(dict(best, nt=nt))
-        if cand['repeat_off']:
-            for nt in cand['nt16']:
-                consider(dict(best, repeat=1, nt=nt))
-        for sb in cand['sb']:
-            consider(dict(best, sb=sb))
+                best, best_ms = dict(fir=k), ms
     finally:
         del x, ph, out, scr
         torch.cuda.empty_cache()
