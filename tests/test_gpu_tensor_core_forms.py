@@ -1,0 +1,130 @@
+"""The tensor-core kernels of the float32 and mixed-precision forms at the sizes where their layouts change: the level's
+product (residues per row, several pulses per unit, partial units and tiles, children in groups, planes of 8 samples,
+short tiles), the float32 form's images against the float64 oracle of the same plan, and the point backprojection's lanes
+per point and the coherence's window forms against plain NumPy."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip('torch')
+if not torch.cuda.is_available():
+    pytest.skip('no CUDA device', allow_module_level=True)
+
+from test_gpu_parity import _level_case, _oracle_level_full, _rel, _run_level_tc, lib  # noqa: E402,F401
+
+
+@pytest.mark.parametrize('case', [
+    # Np, P, K, C, Dk, Dp, frequency pass fraction
+    (5, 37, 60, 4, 2, 2, 0.6),        # a row needs half of the accumulator's rows: two pulses a unit, the last alone
+    (3, 43, 30, 9, 1, 3, 0.6),        # Dk = 1 and 30 columns: four pulses a unit, two groups of 8 child columns
+    (2, 21, 44, 8, 3, 2, 0.6),        # 23 columns, 25 taps
+    (1, 65, 1100, 17, 2, 3, 0.6),     # two residues a row, the last tile's columns odd
+    (1, 33, 515, 3, 1, 1, 0.6),       # no filter on either axis, four columns a row
+    (1, 24, 700, 64, 8, 2, 0.45),     # 8 samples a row, 64 children
+    (1, 40, 500, 64, 11, 3, 0.3),     # two planes of 8 samples
+    (1, 30, 900, 40, 9, 3, 0.45),     # a plane of 8 samples and a gathered one, two steps of it (9 taps a phase)
+    (2, 26, 640, 12, 10, 4, 0.3),     # two gathered planes
+    (1, 20, 1500, 5, 17, 2, 0.2),     # two planes of 8 samples and a gathered one
+], ids=lambda c: 'Np%d-P%d-K%d-C%d-Dk%d-Dp%d' % c[:6])
+def test_level_layouts_match_oracle(lib, oracle_lib, case):  # noqa: F811
+    """The mixed-precision level against the float64 oracle: split float16 products (2^-22) and a float16 intermediate
+    (2^-12 rms a sample, averaged by the pulse filter): below 5e-4."""
+    Np, P, K, C, Dk, Dp, pk = case
+    rng = np.random.default_rng(sum(case[:6]))
+    x, c0, sl, fk, fp, Ko, Po = _level_case(rng, Np, P, K, C, Dk, Dp, pk=pk)
+    got, st = _run_level_tc(lib, x, c0, sl, fk, fp, Ko, Po, Dk, Dp)
+    e = _rel(got, _oracle_level_full(oracle_lib, x, c0, sl, fk, fp, Ko, Po, Dk, Dp))
+    print(f'level {case} Ko {Ko}: rel {e:.2e}')
+    assert st[0] == 0 and e < 5e-4
+
+
+@pytest.mark.parametrize('P,K,nx,ny,T,window', [
+    (97, 83, 33, 65, 16, True),       # odd sizes, T = 16: the last unit of two tiles half empty
+    (128, 96, 64, 64, 32, True),
+    (256, 700, 100, 130, 32, False),  # a first level with long filters
+    (300, 260, 150, 120, 16, True),
+])
+def test_float32_form_matches_float64_oracle(oracle_lib, P, K, nx, ny, T, window):
+    """The float32 former's image against the float64 oracle of the same plan. Per factor float32 rounding, the split
+    float16 products (2^-22) and the hardware sine and cosine (5e-7) leave 1e-6 to 3e-6; the phases here are tens of
+    cycles (float32: 2e-6 rad). Below 1e-5, with the tensor cores in the levels and the final stage."""
+    from fastsar_b200 import ImageFormer, sim
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    rng = np.random.default_rng(P + K)
+    pos, amp = sim.scene(rng, nx, ny, 0.25, 0.25, n_points=12)
+    S = sim.add_noise(sim.simulate_brute(col, pos, amp), 0.01, rng).astype(np.complex64)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, nx, ny, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), T=T, window=window)
+    img = f(S)
+    form, _ = oracle_lib.image_former(col.ant, col.fmin, col.df, K, nx, ny, 0.25, 0.25, e1=(0.0, 1.0, 0.0),
+                                      e2=(1.0, 0.0, 0.0), T=T, window_on=window, kind='port')
+    e = _rel(img, form(S))
+    out = torch.empty((nx, ny), dtype=torch.complex64, device='cuda')
+    kinds = [k for k, _, _ in f._dev.form_profile(torch.from_numpy(S).cuda(), out)]
+    print(f'{P} x {K} -> {nx} x {ny}, T {T}: rel {e:.2e}, {kinds}')
+    assert e < 1e-5
+    assert 'level_tc_gemm' in kinds and kinds[-1] == 'final_tc'
+
+
+def test_float32_form_with_large_phases_keeps_its_kernel(oracle_lib):
+    """A level whose rotation phases pass the bound runs on the CUDA cores (its image is what it was), the later ones on
+    the tensor cores; a non-finite sample is named by either."""
+    from fastsar_b200 import ImageFormer, sim
+    col = sim.spotlight(200, 1500, 9.6e9, 900e6, 20e3, 40.0, 2.0)
+    f = ImageFormer(col.ant, col.fmin, col.df, 1500, 96, 700, 0.3, 0.3, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), T=16)
+    S = torch.randn((200, 1500), dtype=torch.complex64, device='cuda')
+    out = torch.empty((96, 700), dtype=torch.complex64, device='cuda')
+    kinds = [k for k, _, _ in f._dev.form_profile(S, out)]
+    assert kinds[0] == 'level_fp32' and 'level_tc_gemm' in kinds, kinds
+    S[123, 45] = float('nan')
+    with pytest.raises(ValueError, match='pulse 123'):
+        f.form_device(S)
+
+
+@pytest.mark.parametrize('N,P', [(1, 5), (700, 40), (9000, 33), (400000, 3)])
+def test_points_lanes_match_numpy(N, P):
+    """backproject_device at point counts that take 32, some and one lane per point (and fewer pulses than lanes),
+    float64 throughout. The two sides round ranges of 1e4 m (1.8e-12 m) in different orders, 64 cycles a metre: 7e-10
+    rad; below 2e-9."""
+    from fastsar_b200.exact import C, backproject_device
+    rng = np.random.default_rng(N)
+    K, fmin, df = 48, 9.6e9, 2e6
+    ant = np.stack([np.full(P, -7e3), np.linspace(-60, 60, P), np.full(P, 7e3)], 1)
+    S = rng.standard_normal((P, K)) + 1j * rng.standard_normal((P, K))
+    pts = rng.uniform(-20, 20, (N, 3))
+    got = backproject_device(S, ant, fmin, df, pts, window=False, upsample=4).cpu().numpy()
+    nfft, h = 256, K // 2
+    pad = np.zeros((P, nfft), complex)
+    pad[:, :K - h], pad[:, nfft - h:] = S[:, h:], S[:, :h]
+    prof = np.fft.ifft(pad, axis=1) * nfft
+    want = np.zeros(N, complex)
+    for p in range(P):
+        dR = np.linalg.norm(pts - ant[p], axis=1) - np.linalg.norm(ant[p])
+        t = dR * (2 * df * nfft / C)
+        i = np.floor(t).astype(int)
+        w = t - i
+        want += ((1 - w) * prof[p, i % nfft] + w * prof[p, (i + 1) % nfft]) * np.exp(2j * np.pi * (2 * (fmin + h * df) / C) * dR)
+    assert _rel(got, want) < 2e-9
+
+
+@pytest.mark.parametrize('w1,w2', [(1, 3), (2, 2), (5, 7), (8, 3), (11, 10), (12, 5)])
+@pytest.mark.parametrize('n1,n2', [(7, 5), (67, 250)])
+def test_coherence_windows(n1, n2, w1, w2):
+    """The coherence for windows with and without kept rows, images smaller than a window among them, and a strip of
+    zeros (0 there) against float64 window sums: float32 column sums and result, 1e-6."""
+    from scipy.ndimage import uniform_filter
+    from fastsar_b200 import products
+    rng = np.random.default_rng(n1 + w1)
+    a = (rng.standard_normal((n1, n2)) + 1j * rng.standard_normal((n1, n2))).astype(np.complex64)
+    b = (a + rng.standard_normal((n1, n2))).astype(np.complex64)
+    a[:, n2 // 2:n2 // 2 + w2 + 3] = 0
+    A, B = a.astype(complex), b.astype(complex)
+
+    def mean(v):
+        return uniform_filter(v, (w1, w2), mode='nearest')
+    ab = A * B.conj()
+    den = mean(np.abs(A) ** 2) * mean(np.abs(B) ** 2)
+    want = np.sqrt(np.where(den > 1e-20, (mean(ab.real) ** 2 + mean(ab.imag) ** 2) / np.maximum(den, 1e-20), 0.0))
+    got = products.coherence(a, b, w1, w2)
+    zero = mean(np.abs(A) ** 2) < 1e-12
+    np.testing.assert_allclose(got[~zero], want[~zero], rtol=0, atol=2e-6)
