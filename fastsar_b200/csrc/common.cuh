@@ -47,4 +47,36 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
     return d;
 }
 
+// Two float32 values in one 64-bit register: the operands of the packed instructions, kept packed so that no moves
+// rebuild the pairs.
+using f32x2 = unsigned long long;
+
+__device__ __forceinline__ f32x2 pack2(float x, float y)
+{
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 }  // namespace ffbp
