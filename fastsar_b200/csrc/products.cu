@@ -73,26 +73,39 @@ __global__ void __launch_bounds__(256) box_kernel(const void *__restrict__ in, i
 // i - w / 2 + w - 1 along each axis (scipy.ndimage.uniform_filter's placement, fastsar/products.py:35-39). A block
 // of 128 threads owns 128 - (w2 - 1) output columns and a run of rows: each thread keeps the float64 running sums
 // of (Re a b*, Im a b*, |a|^2, |b|^2) over the w1 rows of its column (one row in and one out per output row, fetched
-// an output row ahead of their use); the row's 128 column sums go through shared memory as float32 (16 bytes a
-// column: the shared-memory traffic of the w2-wide sums, which bounds the kernel, halved) to the horizontal sums,
-// and the coherence is formed from those in float64. Rounding the column sums to float32 moves a coherence by about
-// 1e-7.
-constexpr int COH_NT = 128;
+// two output rows ahead of their use); two rows' column sums at a time go through shared memory as float32 (16 bytes a
+// column: half the traffic of the w2-wide sums), where a half of the block takes each row and a thread two neighbouring
+// columns, whose sums share w2 - 1 of their w2 loads; the coherence is formed from those in float64. Rounding the column
+// sums to float32 moves a coherence by about 1e-7. Bound by the conversions to float64 (sixteen a pixel) and issue:
+// 4,097 x 3,911 pixels, 7 x 7 windows, with a 4 x 4 multilook's 47 us: 198 -> 193 us, the same bits (a row at a time, a
+// column per thread before). Runs of 48 rows for windows of up to 8 (repeated on the same images 184 us; 32 / 64 / 128 rows: 185 / 191 / 206 us); longer
+// windows keep 64, since each run starts with the w1 rows of its first window.
+constexpr int COH_NT = 128, COH_ODD = COH_NT / 2 + 4;         // the odd columns' place: 64 bytes off the even ones' banks
+
+// |sum a b*|^2 / (sum |a|^2 sum |b|^2): the windows' 1 / (w1 w2) cancels; the ratio in float64 (the product of two
+// intensity sums can pass float32's range), its square root to float32
+__device__ __forceinline__ float coherence_of(float h0, float h1, float h2, float h3)
+{
+    const double num = (double)h0 * h0 + (double)h1 * h1, den = (double)fmaxf(h2, 0.f) * fmaxf(h3, 0.f);
+    return sqrtf((float)(num / fmax(den, 1e-300)));
+}
 
 __global__ void __launch_bounds__(COH_NT) coherence_kernel(const float2 *__restrict__ a, const float2 *__restrict__ b,
                                                            int n1, int n2, int w1, int w2, int rows,
                                                            float *__restrict__ out)
 {
-    __shared__ float4 sv[COH_NT];
+    // two rows' column sums, even and odd columns apart, twice (the next two rows are written while these are read)
+    __shared__ float4 sv[2][2][COH_ODD + COH_NT / 2 + 1];
     const int t = threadIdx.x, oc = COH_NT - (w2 - 1);
     const int c0 = blockIdx.x * oc, lo1 = w1 / 2, lo2 = w2 / 2;
     const int c = clampi(c0 - lo2 + t, 0, n2 - 1);
     const int rbeg = blockIdx.y * rows, rend = min(rbeg + rows, n1);
+    const float2 *ca = a + c, *cb = b + c;
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     auto fetch = [&](int r, float2 &za, float2 &zb) {
-        const size_t k = (size_t)clampi(r, 0, n1 - 1) * n2 + c;
-        za = a[k];
-        zb = b[k];
+        const size_t k = (size_t)clampi(r, 0, n1 - 1) * n2;
+        za = ca[k];
+        zb = cb[k];
     };
     auto apply = [&](float2 za, float2 zb, double sign) {
         const double ar = za.x, ai = za.y, br = zb.x, bi = zb.y;
@@ -106,32 +119,42 @@ __global__ void __launch_bounds__(COH_NT) coherence_kernel(const float2 *__restr
         fetch(rbeg - lo1 + k, za, zb);
         apply(za, zb, 1.0);
     }
-    // the rows that enter and leave the window at the next slide, fetched an output row ahead of their use
-    float2 ia, ib, xa, xb;
-    fetch(rbeg + 1 - lo1 + w1 - 1, ia, ib);
-    fetch(rbeg - lo1, xa, xb);
-    for (int r = rbeg; r < rend; ++r) {
-        sv[t] = make_float4((float)s0, (float)s1, (float)s2, (float)s3);
+    // the rows that enter and leave the window at the next two slides, fetched ahead of their use
+    float2 ia[2], ib[2], xa[2], xb[2];
+    auto ahead = [&](int r) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            fetch(r + 1 + h - lo1 + w1 - 1, ia[h], ib[h]);
+            fetch(r + h - lo1, xa[h], xb[h]);
+        }
+    };
+    ahead(rbeg);
+    const int slot = (t & 1) * COH_ODD + t / 2, hr = t / (COH_NT / 2), u = t % (COH_NT / 2);
+    for (int r = rbeg, buf = 0; r < rend; r += 2, buf ^= 1) {
+        sv[buf][0][slot] = make_float4((float)s0, (float)s1, (float)s2, (float)s3);
+        apply(ia[0], ib[0], 1.0);
+        apply(xa[0], xb[0], -1.0);
+        sv[buf][1][slot] = make_float4((float)s0, (float)s1, (float)s2, (float)s3);
+        apply(ia[1], ib[1], 1.0);
+        apply(xa[1], xb[1], -1.0);
         __syncthreads();
-        if (t < oc && c0 + t < n2) {
-            float h0 = 0.f, h1 = 0.f, h2 = 0.f, h3 = 0.f;
-            for (int k = 0; k < w2; ++k) {
-                const float4 v = sv[t + k];
+        if (r + 2 < rend) ahead(r + 2);
+        if (r + hr < rend && 2 * u < oc && c0 + 2 * u < n2) {
+            // output columns 2u and 2u + 1 of row r + hr: w2 sums each, w2 - 1 of them shared, in the columns' order
+            const float4 *pe = sv[buf][hr] + u;
+            float g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f, h0 = 0.f, h1 = 0.f, h2 = 0.f, h3 = 0.f;
+            float4 v = pe[0];
+            g0 += v.x; g1 += v.y; g2 += v.z; g3 += v.w;
+            for (int k = 1; k < w2; ++k) {
+                v = pe[(k & 1) * COH_ODD + k / 2];
+                g0 += v.x; g1 += v.y; g2 += v.z; g3 += v.w;
                 h0 += v.x; h1 += v.y; h2 += v.z; h3 += v.w;
             }
-            // |sum a b*|^2 / (sum |a|^2 sum |b|^2): the windows' 1 / (w1 w2) cancels; the ratio in float64 (the
-            // product of two intensity sums can pass float32's range), its square root to float32
-            const double num = (double)h0 * h0 + (double)h1 * h1, den = (double)fmaxf(h2, 0.f) * fmaxf(h3, 0.f);
-            out[(size_t)r * n2 + c0 + t] = sqrtf((float)(num / fmax(den, 1e-300)));
-        }
-        __syncthreads();
-        if (r + 1 < rend) {
-            apply(ia, ib, 1.0);
-            apply(xa, xb, -1.0);
-            if (r + 2 < rend) {
-                fetch(r + 2 - lo1 + w1 - 1, ia, ib);
-                fetch(r + 1 - lo1, xa, xb);
-            }
+            v = pe[(w2 & 1) * COH_ODD + w2 / 2];
+            h0 += v.x; h1 += v.y; h2 += v.z; h3 += v.w;
+            float *o = out + (size_t)(r + hr) * n2 + c0 + 2 * u;
+            o[0] = coherence_of(g0, g1, g2, g3);
+            if (2 * u + 1 < oc && c0 + 2 * u + 1 < n2) o[1] = coherence_of(h0, h1, h2, h3);
         }
     }
 }
@@ -339,7 +362,7 @@ cudaError_t launch_box_mean(const void *in, int kind, int n1, int n2, int w, int
 cudaError_t launch_coherence(const float2 *a, const float2 *b, int n1, int n2, int w1, int w2, float *out,
                              cudaStream_t s)
 {
-    const int oc = COH_NT - (w2 - 1), rows = 64;
+    const int oc = COH_NT - (w2 - 1), rows = w1 <= 8 ? 48 : 64;
     const dim3 grid((n2 + oc - 1) / oc, (n1 + rows - 1) / rows);
     coherence_kernel<<<grid, COH_NT, 0, s>>>(a, b, n1, n2, w1, w2, rows, out);
     return cudaGetLastError();
