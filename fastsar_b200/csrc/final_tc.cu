@@ -4,9 +4,17 @@
 // Each T = 32 tile is the complex sum out[i, j] = sum_n A[i, n] B[j, n] over n = (p, q) (final subaperture p,
 // frequency sample q) with A = d wx exp(-2 pi i ux dlx (a0 + a1 q)) and B = wy exp(-2 pi i uy dly (a0 + a1 q)).
 // As one real product, D = [Ar; Ai] [Br; Bi]^T (64 x 64, K = Pf Qfp with Qf padded to a multiple of 16 by zeros):
-// re = D[i][j] - D[i+32][j+32], im = D[i][j+32] + D[i+32][j].
+// re = D[i][j] - D[i+32][j+32], im = D[i][j+32] + D[i+32][j] (the weighted and the bfloat16 forms).
 //
-// One MMA is M = 128, N = 128, K = 16, and a "unit" is what one accumulator holds:
+// The folded product (float16 and split float16 without aperture weights): rows r and T - 1 - r lie at offsets dl and
+// -dl and columns likewise, so their ramps are conjugates, cos +- i sin. The operands hold the cosine and sine of one
+// row of a pair: A' = [dr cos; di cos; dr sin; di sin] (2 T rows), B' = [cos; sin] (T rows), D = A' B'^T (2 T x T), and the
+// epilogue forms a pair of pairs' four pixels from sums and differences of 8 of its values (tile_fold). Against the full
+// product that is half of B' and of the accumulator, an addition less per value of A', N = 64 instead of 128, and the
+// same roundings per pixel: 107,520 tiles of 36 x 71 in float16 12.46 -> 10.76 ms, 44 x 88 in split float16 27.6 -> 24.8 ms,
+// 4,096 of 40 x 46 696 -> 637 us, 4,320 of 48 x 97 at T = 16 890 -> 837 us.
+//
+// One MMA is M = 128, N = 128 (folded 64), K = 16, and a "unit" is what one accumulator holds:
 //   FFBP_FINAL_TC_BF16X3  one tile, operands split x = hi + lo in bfloat16: A' = [A_hi; A_lo], B' = [B_hi; B_lo], so
 //                         one product gives hi hi, hi lo, lo hi and lo lo of the tile, summed in the epilogue;
 //   the float32 form      one T = 32 or two T = 16 tiles, operands split x = hi + lo in float16 (22 bits; the samples
@@ -14,20 +22,20 @@
 //                         kernel it replaces (images 1.4e-6 to 2.1e-6 against 1.5e-6 to 8.8e-6): the ramps' seeds
 //                         come from the plan as hi + lo, their steps are computed to float32's rounding by the loader
 //                         warp, and the accumulations are cut into short segments (the tensor core's sums truncate).
-//                         4,096 tiles of 40 x 46: 700 us (CUDA cores 1,714); 107,520 of 44 x 88: 27.6 ms (83.9);
-//                         4,320 of 48 x 97 at T = 16: 894 us (2,057). The producers' conversions bound it.
-//   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal 64 x 64
-//                         blocks of the product are the tiles; or four T = 16 tiles, whose 32 x 32 diagonal blocks
-//                         are, each epilogue warp reading one of them from its own lane quarter. The samples are
+//                         4,096 tiles of 40 x 46: 637 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
+//                         4,320 of 48 x 97 at T = 16: 837 us (2,057). The producers' conversions bound it.
+//   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal blocks of the
+//                         product are the tiles; or four T = 16 tiles, the four diagonal blocks, each epilogue warp
+//                         reading one of them from its own lane quarter. The samples are
 //                         scaled by a power of two (from the largest sample component, which the last level kernel
 //                         records) into float16's range, and the pixels by its inverse.
-// The per-instruction issue cost of tcgen05.mma is the same for a 64 x 64 and a 128 x 128 product, so the larger
-// shape does two or four times the work per instruction; two issuing warps double the rate again.
+// M = 128 takes max(32 + N / 4, N / 2) cycles per K step, so the larger shape does two or four times the work per
+// instruction; two issuing warps overlap one's waits on its stage with the other's products.
 //
 // Block roles (persistent over units; one block per SM):
 //   warp 6       loader: stages each final subaperture's samples and geometry by cp.async into a ring of LS
 //                slots, LS - 1 subapertures ahead (its copies' completion arrives on the slot's barrier);
-//   warps 7..18  producers: per final subaperture they build A' and B' (128 rows x Qfp each) in shared memory from
+//   warps 7..18  producers: per final subaperture they build A' and B' (128 and 128 or 64 rows x Qfp) in shared memory from
 //                the staged slot, a row's ramp by a complex recurrence along q seeded in float64, converted to the
 //                operand type, into a ring of S stages (K-major, no swizzle: core matrices of 8 rows x 16 bytes);
 //   warps 4, 5   one thread each issues tcgen05.mma: warp 4 + k takes the final subapertures p = k mod 2 of every
@@ -58,6 +66,8 @@ constexpr int NLD = 1;                     // loader warp 6
 constexpr int NPW = 12;                    // producer warps 7..18
 constexpr int PW0 = NEPI + NISS + NLD;
 constexpr int NTHREADS = (NEPI + NISS + NLD + NPW) * 32;
+constexpr int FS = 6;                      // most stages of folded operands (of the full ones 4): 512-pixel spotlight 36.8
+                                           // against 38.9 us with 4, the larger cases the same
 constexpr int LS = 8;                      // the loader's ring of staged final subapertures
 constexpr int TMEM_COLS = 512;             // NISS issuers x 2 accumulators x 128 columns
 constexpr uint64_t WAIT_NS = 2000000000ull;   // a barrier that has not completed after 2 s counts as stuck
@@ -327,20 +337,66 @@ __device__ __forceinline__ void tile16_pixels(const TcArgs &a, int tile, const f
     }
 }
 
+// The pixels of one tile of the folded operands from its accumulator P (2 TT rows of TT + 1 floats in shared memory; with
+// h = TT / 2 and r, s < h, rows r, h + r, TT + r, TT + h + r: the sums with dr cos, di cos, dr sin, di sin of row r's ramp;
+// columns s, h + s: with the cosine and sine of column s's). Rows r and TT - 1 - r (sg = +-1) and columns s and TT - 1 - s
+// (sj = +-1) are the four sign combinations of d (cx + i sg sx) (cy + i sj sy). Thread t of 2 TT h / 8 takes row pair
+// t / (TT / 4) and two neighbouring column pairs: 8 pixels, whose quadratic phases are equal in twos.
+template <int TT>
+__device__ __forceinline__ void tile_fold(const TcArgs &a, int tile, const float *P, int t, float scale)
+{
+    constexpr int h = TT / 2, W = TT + 1;
+    const int r = t / (TT / 4), s0 = 2 * (t % (TT / 4));
+    const double cx = a.ucx[tile], cy = a.ucy[tile];
+    const float f = (float)(a.fc2 / (2.0 * a.rc[tile]));
+    const float dx = ((float)r - 0.5f * (TT - 1)) * (float)a.spx;
+    const int2 f0 = a.img ? a.first[tile] : make_int2(0, 0);
+    const float *p0 = P + r * W + s0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int s = s0 + k;
+        const float ccr = p0[k], csr = p0[h + k], cci = p0[h * W + k], csi = p0[h * W + h + k];
+        const float scr = p0[TT * W + k], ssr = p0[TT * W + h + k];
+        const float sci = p0[(TT + h) * W + k], ssi = p0[(TT + h) * W + h + k];
+        const float dy = ((float)s - 0.5f * (TT - 1)) * (float)a.spy;
+#pragma unroll
+        for (int opp = 0; opp < 2; ++opp) {                    // sg == sj, then sg == -sj
+            const float los = opp ? (float)cx * dx - (float)cy * dy : (float)cx * dx + (float)cy * dy;
+            const float2 e = cis_cycles((dx * dx + dy * dy - los * los) * f);
+            const float er = opp ? ccr + ssr : ccr - ssr, ei = opp ? cci + ssi : cci - ssi;
+            const float dr = opp ? csi - sci : csi + sci, di = opp ? csr - scr : csr + scr;
+#pragma unroll
+            for (int neg = 0; neg < 2; ++neg) {                 // sj = +1, then -1
+                const int j = neg ? TT - 1 - s : s, i = (neg != 0) != (opp != 0) ? TT - 1 - r : r;
+                const float2 o = cmul(make_float2(neg ? er + dr : er - dr, neg ? ei - di : ei + di), e);
+                const float2 ov = make_float2(o.x * scale, o.y * scale);
+                if (a.img) {
+                    const int x = f0.x + i - a.ox, y = f0.y + j - a.oy;
+                    if (x >= 0 && x < a.nx && y >= 0 && y < a.ny) a.img[(size_t)x * a.ny + y] = ov;
+                } else {
+                    a.tiles[((size_t)tile * TT + i) * TT + j] = ov;
+                }
+            }
+        }
+    }
+}
+
 template <int OP, bool WEIGHTED, int MAXWI, int TT>
 __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
 {
-    constexpr bool BF = OP == OP_BF16X2, X2 = OP == OP_F16X2;
+    constexpr bool BF = OP == OP_BF16X2, X2 = OP == OP_F16X2, FOLD = !BF && !WEIGHTED;
+    constexpr int NB = FOLD ? 64 : 128;                         // operand rows of B': the accumulator's columns
     constexpr int NTS = unit_tiles<OP, TT>();                   // tiles per unit
     extern __shared__ __align__(1024) unsigned char smem[];
     const int ng = a.Qfp / 8;                                   // core matrices along K per operand
     const uint32_t H = 64u * a.Qfp * 2u;                        // 64 operand rows
     const uint32_t HS = 2u * TT * a.Qfp * 2u;                   // one part (hi or lo) of a tile's operand rows, 2 TT rows
-    const uint32_t stagebytes = 4u * H;                         // A' (128 rows), B' (128 rows)
-    float *sP = reinterpret_cast<float *>(smem + (size_t)a.S * stagebytes);             // [2][32][65]
+    const uint32_t HB = FOLD ? HS / 2 : HS;                     // a part of a tile's rows of B'
+    const uint32_t stagebytes = FOLD ? 3u * H : 4u * H;         // A' (128 rows), B' (NB rows)
+    float *sP = reinterpret_cast<float *>(smem + (size_t)a.S * stagebytes);             // [2][32][65] or [2][64][33]
     // the loader's ring: per slot and tile slot, the subaperture's Qfp samples (zero past Qf), ux, uy and the
     // three weights (split float16: the seeds of both ramps and the steps of the TT / 2 row pairs of each); tsb bytes
-    unsigned char *ring = reinterpret_cast<unsigned char *>(sP + 2 * 32 * 65);
+    unsigned char *ring = reinterpret_cast<unsigned char *>(sP + (FOLD ? 2 * 64 * 33 : 2 * 32 * 65));
     const uint32_t tsb = 8u * a.Qfp + 32u + (X2 ? 8u * TT : 0u), slotbytes = (uint32_t)NTS * tsb;
     uint64_t *bars = reinterpret_cast<uint64_t *>(ring + (size_t)LS * slotbytes);
     uint64_t *full = bars, *empty = bars + a.S, *accf = bars + 2 * a.S, *acce = accf + 2, *drain = acce + 2;
@@ -479,7 +535,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         const int r = lane % (TT / 2), sub = lane / (TT / 2);
         uint32_t roff[4];
         {
-            const int rows[4] = {r, r + TT, TT - 1 - r, 2 * TT - 1 - r};
+            const int rows[4] = {r, r + TT / 2, r + TT, r + TT + TT / 2};
 #pragma unroll
             for (int k = 0; k < 4; ++k) roff[k] = (uint32_t)(((rows[k] >> 3) * ng) * 128 + (rows[k] & 7) * 16);
         }
@@ -507,7 +563,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     c1 -= rintf(c1);
                     float2 wv = cis_cycles(-((c0 + c1) + fmaf(m, sd.y, n8 * sd.w)));
                     const float2 st = *reinterpret_cast<const float2 *>(tsp + 8 * a.Qfp + 32 + 8 * ((isA ? 0 : TT / 2) + r));
-                    unsigned char *ob = smem + (size_t)stg * stagebytes + (isA ? 0u : 2u * H) + (uint32_t)ts * (2u * HS) + (uint32_t)g * 128u;
+                    const uint32_t part = isA ? HS : HB;
+                    unsigned char *ob = smem + (size_t)stg * stagebytes + (isA ? 0u : 2u * H) + (uint32_t)ts * (2u * part) + (uint32_t)g * 128u;
                     uint4 h, l;
                     if (isA) {
                         wv.x *= dscale;
@@ -521,9 +578,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                             for (int hh = 0; hh < 2; ++hh) {
                                 const int e = 2 * e2 + hh;
                                 const float dr = hh ? dd.z : dd.x, di = hh ? dd.w : dd.y;
-                                const float pr = dr * wv.x, pi = di * wv.x;
-                                r1[e] = fmaf(-di, wv.y, pr); i1[e] = fmaf(dr, wv.y, pi);   // d x
-                                r2[e] = fmaf(di, wv.y, pr); i2[e] = fmaf(-dr, wv.y, pi);   // d conj(x)
+                                r1[e] = dr * wv.x; i1[e] = di * wv.x;
+                                r2[e] = dr * wv.y; i2[e] = di * wv.y;
                                 wv = cmul(wv, st);
                             }
                         }
@@ -549,14 +605,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                         }
                         pack8<OP>(r1, h, l);
                         *reinterpret_cast<uint4 *>(ob + roff[0]) = h;
-                        *reinterpret_cast<uint4 *>(ob + HS + roff[0]) = l;
-                        *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
-                        *reinterpret_cast<uint4 *>(ob + HS + roff[2]) = l;
+                        *reinterpret_cast<uint4 *>(ob + HB + roff[0]) = l;
                         pack8<OP>(i1, h, l);
                         *reinterpret_cast<uint4 *>(ob + roff[1]) = h;
-                        *reinterpret_cast<uint4 *>(ob + HS + roff[1]) = l;
-                        *reinterpret_cast<uint4 *>(ob + roff[3]) = flip_sign(h);
-                        *reinterpret_cast<uint4 *>(ob + HS + roff[3]) = flip_sign(l);
+                        *reinterpret_cast<uint4 *>(ob + HB + roff[1]) = l;
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -580,9 +632,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         // ------------------------------------------------------------------ producers
         // Warp items: (tile slot ts, operand A or B, pair of 8-sample groups gp). Lane l of the warp takes pixel
         // row pair r = l % 16 (rows r and 31 - r, whose offsets are dl and -dl, so that their ramps are complex
-        // conjugates and one recurrence serves both) and group g = 2 gp + l / 16. An A item writes Ar, Ai of rows
-        // r and 31 - r (d times the ramp and d times its conjugate); a B item writes Br, Bi of row r and, without
-        // weights, row 31 - r from row r's words (the same real part, the imaginary part's sign flipped).
+        // conjugates and one recurrence serves both) and group g = 2 gp + l / 16. Folded, an A item writes dr and di times
+        // the ramp's cosine and sine, a B item its cosine and sine. Otherwise an A item writes Ar, Ai of rows r and
+        // 31 - r (d times the ramp and d times its conjugate), a B item Br, Bi of row r and, without weights, row
+        // 31 - r from row r's words (the same real part, the imaginary part's sign flipped).
         const int pw = warp - PW0;
         constexpr int GPI = 64 / TT;                            // 8-sample groups per item: a lane per row pair
         const int hg = (ng + GPI - 1) / GPI;
@@ -593,7 +646,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         // byte offsets (without the group) of rows r, r + TT, TT - 1 - r, 2 TT - 1 - r within a tile's 2 TT rows
         uint32_t roff[4];
         {
-            const int rows[4] = {r, r + TT, TT - 1 - r, 2 * TT - 1 - r};
+            const int rows[4] = {r, FOLD ? r + TT / 2 : r + TT, FOLD ? r + TT : TT - 1 - r, FOLD ? r + TT + TT / 2 : 2 * TT - 1 - r};
 #pragma unroll
             for (int k = 0; k < 4; ++k) roff[k] = (uint32_t)(((rows[k] >> 3) * ng) * 128 + (rows[k] & 7) * 16);
         }
@@ -668,7 +721,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     else { w1 = 1.f + gw[2] * dlf; w2 = 1.f - gw[2] * dlf; }
                 }
                 // operand base: A' or B'; half: bfloat16 hi (lo one half further), float16 the tile slot's; group g
-                unsigned char *ob = sbase + (isA ? 0u : 2u * H) + (BF ? 0u : (uint32_t)ts * HS) + (uint32_t)g * 128u;
+                unsigned char *ob = sbase + (isA ? 0u : 2u * H) + (BF ? 0u : (uint32_t)ts * (isA ? HS : HB)) + (uint32_t)g * 128u;
                 float r1[8], i1[8], r2[8], i2[8];
                 if (isA) {
                     const float4 *dq = reinterpret_cast<const float4 *>(tsp + 64 * g);
@@ -680,6 +733,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                             const int e = 2 * e2 + h;
                             const float dr = h ? dd.z : dd.x, di = h ? dd.w : dd.y;
                             const float p1 = dr * wv.x, p2 = di * wv.y, p3 = dr * wv.y, p4 = di * wv.x;
+                            if (FOLD) {
+                                r1[e] = p1; i1[e] = p4; r2[e] = p3; i2[e] = p2;
+                                wv = cmul(wv, st);
+                                continue;
+                            }
                             r1[e] = (p1 - p2) * w1; i1[e] = (p3 + p4) * w1;       // d x
                             r2[e] = (p1 + p2) * w2; i2[e] = (p4 - p3) * w2;       // d conj(x)
                             wv = cmul(wv, st);
@@ -695,7 +753,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     }
                 }
                 uint4 h, l;
-                const bool mirror = !isA && !WEIGHTED;
+                const bool mirror = !isA && !WEIGHTED && !FOLD, half = !isA && FOLD;
                 pack8<OP>(r1, h, l);
                 *reinterpret_cast<uint4 *>(ob + roff[0]) = h;
                 if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[0]) = l;
@@ -709,7 +767,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 if (mirror) {
                     *reinterpret_cast<uint4 *>(ob + roff[3]) = flip_sign(h);
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[3]) = flip_sign(l);
-                } else {
+                } else if (!half) {
                     pack8<OP>(r2, h, l);
                     *reinterpret_cast<uint4 *>(ob + roff[2]) = h;
                     if (BF) *reinterpret_cast<uint4 *>(ob + H + roff[2]) = l;
@@ -736,7 +794,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
         // ------------------------------------------------------------------ MMA issue
         const int k = warp - NEPI;
         if (lane == 0 && k < nis) {
-            const uint32_t idesc = (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | ((128u >> 3) << 17) |
+            const uint32_t idesc = (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | (((uint32_t)NB >> 3) << 17) |
                                    ((128u >> 4) << 24);
             const uint32_t lbo = 128, sbo = (uint32_t)ng * 128;
             const int nks = a.Qfp / 16;
@@ -792,11 +850,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 // The tensor core's float32 sums truncate: a chain of n of them loses about n 3e-8 of the result. So a
                 // unit is accumulated in segments, added here in float32 with rounding. This thread's accumulator row,
                 // hi and lo columns summed:
-                constexpr int NV = TT == 32 ? 64 : 32;
+                constexpr int NV = TT;
                 float v[NV];
 #pragma unroll
                 for (int i = 0; i < NV; ++i) v[i] = 0.f;
-                const int c0 = TT == 32 ? 0 : 64 * (warp >> 1);
+                const int c0 = TT == 32 ? 0 : 32 * (warp >> 1);
                 for (int sg = 0; sg < a.nsg; ++sg, ++j) {
                     const int ab = j & 1, na = min(nis, a.Pf - sg * a.seg);   // issuers with a stage in the segment
                     if (live) live = mbar_wait<EPILOGUE_HINT_NS>(&accf[ab], (uint32_t)((j >> 1) & 1), &s_abort, a.err);
@@ -821,21 +879,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 }
                 if (TT == 32) {
                     // warps 0, 1: the hi rows; then warps 2, 3 add the lo rows
+                    float *part = sP + ((warp & 1) * 32 + lane) * (TT + 1);
                     if (live && warp < 2) {
 #pragma unroll
-                        for (int i = 0; i < NV; ++i) mine[lane * 65 + i] = v[i];
+                        for (int i = 0; i < NV; ++i) part[i] = v[i];
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (live && warp >= 2) {
 #pragma unroll
-                        for (int i = 0; i < NV; ++i) mine[lane * 65 + i] += v[i];
+                        for (int i = 0; i < NV; ++i) part[i] += v[i];
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (live) tile_pixels(a, unit_tile<OP, TT>(ul, 0), P0, P1, t, oscale);
+                    if (live) tile_fold<TT>(a, unit_tile<OP, TT>(ul, 0), sP, t, oscale);
                 } else {
-                    // tile slot ts = warp / 2: the hi rows (Re, Im) in the even warp's lanes, the lo rows in the odd one's
-                    const int ts = warp >> 1;
-                    float *part = sP + ts * (32 * 33) + lane * 33;
+                    // tile slot ts = warp / 2: the hi rows in the even warp's lanes, the lo rows in the odd one's
+                    const int ts = warp >> 1, tile = unit_tile<OP, TT>(ul, ts);
+                    float *part = sP + ts * (32 * (TT + 1)) + lane * (TT + 1);
                     if (live && (warp & 1)) {
 #pragma unroll
                         for (int i = 0; i < NV; ++i) part[i] = v[i];
@@ -843,8 +902,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (live && !(warp & 1)) {
 #pragma unroll
-                        for (int i = 0; i < NV; ++i) v[i] += part[i];
-                        tile16_pixels(a, unit_tile<OP, TT>(ul, ts), v, v + 16, lane, oscale);
+                        for (int i = 0; i < NV; ++i) part[i] += v[i];
+                        __syncwarp();
+                        if (tile < a.B) tile_fold<TT>(a, tile, sP + ts * (32 * (TT + 1)), lane, oscale);
                     }
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -896,6 +956,44 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (live) tile_pixels(a, unit_tile<OP, TT>(ul, 0), P0, P1, t, oscale);
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            } else if (FOLD && TT == 16) {
+                // tile slot ts = warp: accumulator rows [32 ts, 32 ts + 32) (this warp's lane quarter) at columns
+                // [16 ts, 16 ts + 16)
+                if (live) {
+                    float v[16], *part = sP + warp * (32 * (TT + 1));
+                    gather(16 * warp, 0, v);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acce[ab]);
+                    const int tile = unit_tile<OP, TT>(ul, warp);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) part[lane * (TT + 1) + i] = v[i];
+                    __syncwarp();
+                    if (tile < a.B) tile_fold<TT>(a, tile, part, lane, oscale);
+                    __syncwarp();
+                }
+            } else if (FOLD) {
+                // tile slot ts: accumulator rows [64 ts, 64 ts + 64) and columns [32 ts, 32 ts + 32), read by warps 2 ts and
+                // 2 ts + 1
+                const int ts = warp >> 1;
+                if (live) {
+                    float v[16], *part = sP + (ts * 64 + (warp & 1) * 32 + lane) * (TT + 1);
+#pragma unroll
+                    for (int c0 = 0; c0 < 32; c0 += 16) {
+                        gather(32 * ts + c0, 0, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) part[c0 + i] = v[i];
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acce[ab]);
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                for (int k = 0; k < 2; ++k) {
+                    const int tile = unit_tile<OP, TT>(ul, k);
+                    if (live && tile < a.B) tile_fold<TT>(a, tile, sP + k * 64 * (TT + 1), t, oscale);
+                }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             } else if (TT == 16) {
                 // tile slot ts = warp: accumulator rows [32 ts, 32 ts + 32) (this warp's lane quarter) at columns
@@ -1004,7 +1102,7 @@ namespace {
 struct TcShape { int nts, nwi, maxwi, S; size_t smem; };
 
 // The unit and the ring of a final stage's shape (op: Operands); false with *why for shapes the kernel does not cover.
-bool tc_shape(int op, int T, int Pf, int Qf, size_t maxsmem, TcShape *o, const char **why)
+bool tc_shape(int op, bool weighted, int T, int Pf, int Qf, size_t maxsmem, TcShape *o, const char **why)
 {
     const bool split = op != OP_F16;
     if (T != 32 && (T != 16 || op == OP_BF16X2)) {
@@ -1031,6 +1129,12 @@ bool tc_shape(int op, int T, int Pf, int Qf, size_t maxsmem, TcShape *o, const c
     }
     o->S = S;
     o->smem = (size_t)S * stage + fixed;
+    if (op != OP_BF16X2 && !weighted) {                         // folded operands: three quarters of a stage (what fits is
+        const size_t st3 = stage / 4 * 3, fx3 = fixed + 2 * 64 * 4 + (2 * FS - 8) * 8;   // decided above, as before)
+        for (S = FS; S > 2 && ((size_t)S * st3 + fx3 > avail || S % nis); --S) {}
+        o->S = S;
+        o->smem = (size_t)S * st3 + fx3;
+    }
     return true;
 }
 
@@ -1048,7 +1152,7 @@ bool final_tc32_supported(int T, int B, int Pf, int Qf)
 {
     const char *why = nullptr;
     TcShape o;
-    return (long long)B * Pf < (1LL << 31) && tc_shape(OP_F16X2, T, Pf, Qf, max_smem(), &o, &why);
+    return (long long)B * Pf < (1LL << 31) && tc_shape(OP_F16X2, false, T, Pf, Qf, max_smem(), &o, &why);
 }
 
 cudaError_t launch_final_tc(const FinalLaunch &F, int mode, cudaStream_t s, const char **why)
@@ -1056,7 +1160,7 @@ cudaError_t launch_final_tc(const FinalLaunch &F, int mode, cudaStream_t s, cons
     *why = nullptr;
     const int op = mode == 0 ? OP_F16X2 : (mode == 2 ? OP_BF16X2 : OP_F16);
     TcShape o;
-    if (!tc_shape(op, F.T, F.Pf, F.Qf, max_smem(), &o, why)) return cudaErrorNotSupported;
+    if (!tc_shape(op, F.w != nullptr, F.T, F.Pf, F.Qf, max_smem(), &o, why)) return cudaErrorNotSupported;
     if (F.B <= 0) return cudaSuccess;
     if ((long long)F.B * F.Pf >= (1LL << 31)) { *why = "more than 2^31 final tile subapertures"; return cudaErrorNotSupported; }
     TcArgs a;
