@@ -33,9 +33,9 @@
 // instruction; two issuing warps overlap one's waits on its stage with the other's products.
 //
 // Block roles (persistent over units; one block per SM):
-//   warp 6       loader: stages each final subaperture's samples and geometry by cp.async into a ring of LS
+//   warp 6, 7    loaders, one or two that alternate (loaders): stage each final subaperture's samples and geometry by cp.async into a ring of LS
 //                slots, LS - 1 subapertures ahead (its copies' completion arrives on the slot's barrier);
-//   warps 7..18  producers: per final subaperture they build A' and B' (128 and 128 or 64 rows x Qfp) in shared memory from
+//   12 warps after them  producers: per final subaperture they build A' and B' (128 and 128 or 64 rows x Qfp) in shared memory from
 //                the staged slot, a row's ramp by a complex recurrence along q seeded in float64, converted to the
 //                operand type, into a ring of S stages (K-major, no swizzle: core matrices of 8 rows x 16 bytes);
 //   warps 4, 5   one thread each issues tcgen05.mma: warp 4 + k takes the final subapertures p = k mod 2 of every
@@ -62,10 +62,7 @@ namespace {
 
 constexpr int NEPI = 4;                    // epilogue warps 0..3 (TMEM lane quarters 0..3)
 constexpr int NISS = 2;                    // MMA issuing warps 4, 5
-constexpr int NLD = 1;                     // loader warp 6
-constexpr int NPW = 12;                    // producer warps 7..18
-constexpr int PW0 = NEPI + NISS + NLD;
-constexpr int NTHREADS = (NEPI + NISS + NLD + NPW) * 32;
+constexpr int NPW = 12;                    // producer warps, after the loaders
 constexpr int FS = 6;                      // most stages of folded operands (of the full ones 4): 512-pixel spotlight 36.8
                                            // against 38.9 us with 4, the larger cases the same
 constexpr int LS = 8;                      // the loader's ring of staged final subapertures
@@ -251,6 +248,23 @@ __device__ __forceinline__ uint4 flip_sign(uint4 v)
     return make_uint4(v.x ^ sg, v.y ^ sg, v.z ^ sg, v.w ^ sg);
 }
 
+// Loader warps (6, or 6 and 7). Of the folded forms one warp's copies bound the stages (a subaperture of 33 x 37 took 700 ns,
+// the producers 500), so two take turns: 2,048 x 2,048 pixels 637 -> 512 us in the float32 form and 367 -> 268 us in
+// float16, 1,499 x 701 at T = 16 837 -> 754 and 573 -> 483 us. Two items of T = 32 in float16 per producer warp take longer
+// than their copies, and the block with a 20th warp runs them slower, with one loader at work or two (107,520 tiles of
+// 36 x 71: 10.75 ms with one, 12.1 with two; 900 of 72 x 96: 268 and 272 us); from three on two gain again (2,400 of
+// 82 x 126: 985 -> 951 us).
+template <int OP, bool WEIGHTED, int MAXWI, int TT> __host__ __device__ constexpr int loaders()
+{
+    return OP == OP_BF16X2 || WEIGHTED || (OP == OP_F16 && TT == 32 && MAXWI == 2) ? 1 : 2;
+}
+
+// Threads of a block.
+template <int OP, bool WEIGHTED, int MAXWI, int TT> __host__ __device__ constexpr int block_threads()
+{
+    return (NEPI + NISS + loaders<OP, WEIGHTED, MAXWI, TT>() + NPW) * 32;
+}
+
 // Tiles per unit: 128 operand rows hold 2 TT rows per tile, twice that when split.
 template <int OP, int TT> __host__ __device__ constexpr int unit_tiles() { return OP == OP_F16 ? 64 / TT : 32 / TT; }
 
@@ -382,8 +396,10 @@ __device__ __forceinline__ void tile_fold(const TcArgs &a, int tile, const float
 }
 
 template <int OP, bool WEIGHTED, int MAXWI, int TT>
-__global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
+__global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) final_tc_kernel(const TcArgs a)
 {
+    constexpr int NLD = loaders<OP, WEIGHTED, MAXWI, TT>(), PW0 = NEPI + NISS + NLD;
+    constexpr int NTHREADS = block_threads<OP, WEIGHTED, MAXWI, TT>();
     constexpr bool BF = OP == OP_BF16X2, X2 = OP == OP_F16X2, FOLD = !BF && !WEIGHTED;
     constexpr int NB = FOLD ? 64 : 128;                         // operand rows of B': the accumulator's columns
     constexpr int NTS = unit_tiles<OP, TT>();                   // tiles per unit
@@ -444,7 +460,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
     const uint32_t tmem = s_tmem;
     const uint32_t smem0 = smem_u32(smem);
 
-    if (warp == NEPI + NISS) {
+    if (warp >= NEPI + NISS && warp < PW0) {
         // ------------------------------------------------------------------ loader
         // Stages every final subaperture of this block's units LS - 1 ahead of the producers: per tile slot the
         // Qfp samples (8 bytes each, zero past Qf and for a tile past the last), ux, uy and the weights, by cp.async
@@ -471,7 +487,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     asm volatile("prefetch.global.L2 [%0];" :: "l"(src + o));
             }
         };
-        int ul = 0, p = 0;
+        // loader k takes every NLD-th subaperture from the k-th on: ul, p its unit and subaperture
+        const int k0 = warp - (NEPI + NISS);
+        int ul = k0 / a.Pf, p = k0 % a.Pf;
         // split float16: lane l computes the step of row pair r of operand xop of tile slot xts, whose slope it reads
         // a subaperture ahead
         const int xts = X2 ? lane / TT : 0, xop = (lane % TT) / (TT / 2), xr = lane % (TT / 2);
@@ -482,8 +500,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
             if (tile < a.B)
                 slope = *(reinterpret_cast<const float2 *>(a.seeds + 2 * ((size_t)tile * a.Pf + fp) + xop) + 1);
         };
-        if (X2) fetch_slope(0, 0);
-        for (int it = 0; it < ntot; ++it) {
+        if (X2) fetch_slope(ul, p);
+        for (int it = k0; it < ntot; it += NLD) {
             const int ls = it % LS;
             if (it >= LS && !mbar_wait<PRODUCER_HINT_NS>(&lempty[ls], (uint32_t)((it / LS - 1) & 1), &s_abort, a.err))
                 break;
@@ -509,7 +527,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) final_tc_kernel(const TcArgs a)
                     cp_async(gd + 16u + 4u * (lane - 2), (const void *)(a.w + (size_t)(lane - 2) * nbp + bp), 4, tv);
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&lfull[ls])) : "memory");
-            if (++p == a.Pf) { p = 0; ++ul; }
+            for (p += NLD; p >= a.Pf; p -= a.Pf) ++ul;
             if (X2) {
                 const float m = (float)(2 * xr - (TT - 1));
                 float c = m * slope.x;                          // exact; the low part then moves it by a rounding
@@ -1183,23 +1201,25 @@ cudaError_t launch_final_tc(const FinalLaunch &F, int mode, cudaStream_t s, cons
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int grid = a.nunits < nsm ? a.nunits : nsm;
-    auto run = [&](auto kern) -> cudaError_t {
+    auto run = [&](auto kern, int threads) -> cudaError_t {
         cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o.smem);
         if (r != cudaSuccess) return r;
-        kern<<<grid, NTHREADS, o.smem, s>>>(a);
+        kern<<<grid, threads, o.smem, s>>>(a);
         return cudaGetLastError();
     };
+#define FFBP_TC_ONE(OP, W, MW, TT) run(final_tc_kernel<OP, W, MW, TT>, block_threads<OP, W, MW, TT>())
     if (op == OP_F16X2) {
         // weighted tiles: a pulse's weight has no bound that float16's range could be held to
         if (a.w || !a.seeds) { *why = "the split float16 final stage takes the plan's seeds and no aperture weights"; return cudaErrorNotSupported; }
-        return F.T == 16 ? run(final_tc_kernel<OP_F16X2, false, 1, 16>) : run(final_tc_kernel<OP_F16X2, false, 1, 32>);
+        return F.T == 16 ? FFBP_TC_ONE(OP_F16X2, false, 1, 16) : FFBP_TC_ONE(OP_F16X2, false, 1, 32);
     }
-#define FFBP_TC_RUN(MW)                                                                                       \
-    (op == OP_BF16X2 ? (a.w ? run(final_tc_kernel<OP_BF16X2, true, MW, 32>) : run(final_tc_kernel<OP_BF16X2, false, MW, 32>)) \
-     : F.T == 16     ? (a.w ? run(final_tc_kernel<OP_F16, true, MW, 16>) : run(final_tc_kernel<OP_F16, false, MW, 16>))   \
-                     : (a.w ? run(final_tc_kernel<OP_F16, true, MW, 32>) : run(final_tc_kernel<OP_F16, false, MW, 32>)))
+#define FFBP_TC_RUN(MW)                                                                                         \
+    (op == OP_BF16X2 ? (a.w ? FFBP_TC_ONE(OP_BF16X2, true, MW, 32) : FFBP_TC_ONE(OP_BF16X2, false, MW, 32))          \
+     : F.T == 16     ? (a.w ? FFBP_TC_ONE(OP_F16, true, MW, 16) : FFBP_TC_ONE(OP_F16, false, MW, 16))                \
+                     : (a.w ? FFBP_TC_ONE(OP_F16, true, MW, 32) : FFBP_TC_ONE(OP_F16, false, MW, 32)))
     return o.maxwi <= 1 ? FFBP_TC_RUN(1) : o.maxwi <= 2 ? FFBP_TC_RUN(2) : FFBP_TC_RUN(4);
 #undef FFBP_TC_RUN
+#undef FFBP_TC_ONE
 }
 
 }  // namespace ffbp
