@@ -22,8 +22,8 @@
 //                         kernel it replaces (images 1.4e-6 to 2.1e-6 against 1.5e-6 to 8.8e-6): the ramps' seeds
 //                         come from the plan as hi + lo, their steps are computed to float32's rounding by the loader
 //                         warp, and the accumulations are cut into short segments (the tensor core's sums truncate).
-//                         4,096 tiles of 40 x 46: 637 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
-//                         4,320 of 48 x 97 at T = 16: 837 us (2,057). The producers' conversions bound it.
+//                         4,096 tiles of 40 x 46: 512 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
+//                         4,320 of 48 x 97 at T = 16: 754 us (2,057). The producers' conversions bound it.
 //   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal blocks of the
 //                         product are the tiles; or four T = 16 tiles, the four diagonal blocks, each epilogue warp
 //                         reading one of them from its own lane quarter. The samples are
