@@ -22,8 +22,8 @@
 //                         kernel it replaces (images 1.4e-6 to 2.1e-6 against 1.5e-6 to 8.8e-6): the ramps' seeds
 //                         come from the plan as hi + lo, their steps are computed to float32's rounding by the loader
 //                         warp, and the accumulations are cut into short segments (the tensor core's sums truncate).
-//                         4,096 tiles of 40 x 46: 512 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
-//                         4,320 of 48 x 97 at T = 16: 754 us (2,057). The producers' conversions bound it.
+//                         4,096 tiles of 40 x 46: 533 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
+//                         4,320 of 48 x 97 at T = 16: 714 us (2,057). The producers' conversions bound it.
 //   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal blocks of the
 //                         product are the tiles; or four T = 16 tiles, the four diagonal blocks, each epilogue warp
 //                         reading one of them from its own lane quarter. The samples are
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
     if (t == 0) {
         s_abort = 0;
         for (int s = 0; s < a.S; ++s) {
-            mbar_init(&full[s], X2 ? (uint32_t)a.nwi : NPW);
+            mbar_init(&full[s], NPW);
             mbar_init(&empty[s], 1);
         }
         for (int k = 0; k < 2; ++k) {
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
         for (int k = 0; k < LS; ++k) {
             // the loader's 32 threads, once their copies have landed (split float16: and their steps are written)
             mbar_init(&lfull[k], X2 ? 64 : 32);
-            mbar_init(&lempty[k], X2 ? (uint32_t)a.nwi : NPW);
+            mbar_init(&lempty[k], NPW);
         }
         mbar_init(&s_never, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -544,9 +544,13 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
     } else if (X2 && warp >= PW0) {
         // ------------------------------------------------------------------ producers, split float16
         // Items, lanes and rows as below. Here the items (twice the conversions and stores) alternate A, the heavier,
-        // and B, and are dealt to the warps in turn from a start that moves by one more than their count per stage: every
-        // warp gets as many of each and runs ahead over the ring (a stage is full once its nwi items have arrived; a
-        // fixed set of items per warp and stage was 1.4 times slower at 40 x 46).
+        // and B, and are dealt to the warps in turn from a start that moves by one more than their count per stage, so
+        // that the warps' loads even out over a few stages (a fixed set of items per warp and stage was 1.4 times slower
+        // at 40 x 46). With fewer items than warps some have none in a subaperture: they wait and arrive with the others
+        // all the same. A parity wait tells a phase from its neighbours only: a warp that skipped one could test a slot
+        // or a stage two phases ahead of its barrier (and pass), and one that waited without arriving could be passed
+        // by two phases (and wait for ever). With the waits left out where there was no item 4,096 tiles of 40 x 46 took 512 us,
+        // with them 533; one arrival a warp instead of one an item 754 -> 714 us (4,320 of 48 x 97 at T = 16).
         const int pw = warp - PW0;
         constexpr int GPI = 64 / TT;
         const int ngr = (a.Qf + 7) / 8, hg = (ngr + GPI - 1) / GPI, ntot = nul * a.Pf;
@@ -563,10 +567,8 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
         uint32_t pp0 = 0, pp1 = 0;
         for (int it = 0; it < ntot; ++it) {
             const int ls = it % LS, kq = nis == 2 ? (p & 1) : 0, stg = kq + nis * (kq ? ps1 : ps0);
-            if (first < a.nwi &&
-                !(mbar_wait<PRODUCER_HINT_NS>(&lfull[ls], (uint32_t)((it / LS) & 1), &s_abort, a.err) &&
-                  mbar_wait<PRODUCER_HINT_NS>(&empty[stg], (kq ? pp1 : pp0) ^ 1u, &s_abort, a.err)))
-                break;
+            if (!mbar_wait<PRODUCER_HINT_NS>(&lfull[ls], (uint32_t)((it / LS) & 1), &s_abort, a.err)) break;
+            if (!mbar_wait<PRODUCER_HINT_NS>(&empty[stg], (kq ? pp1 : pp0) ^ 1u, &s_abort, a.err)) break;
             for (int item = first; item < a.nwi; item += NPW) {
                 const int q = item >> 1, ts = NTS == 1 ? 0 : q / hg, g = GPI * (NTS == 1 ? q : q - ts * hg) + sub;
                 const bool isA = (item & 1) == 0;
@@ -629,12 +631,12 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
                         *reinterpret_cast<uint4 *>(ob + HB + roff[1]) = l;
                     }
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&full[stg]);
-                    mbar_arrive(&lempty[ls]);
-                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&full[stg]);
+                mbar_arrive(&lempty[ls]);
             }
             first -= turn;
             if (first < 0) first += NPW;

@@ -66,6 +66,40 @@ def test_float32_form_matches_float64_oracle(oracle_lib, P, K, nx, ny, T, window
     assert 'level_tc_gemm' in kinds and kinds[-1] == 'final_tc'
 
 
+@pytest.mark.parametrize('P,K,bw,ap,sp,T,items,odd', [
+    (200, 16, 20e6, 1.5, 0.25, 32, 2, True),       # final subapertures of 2, 4 and 6 items for the twelve warps that
+    (201, 16, 20e6, 1.5, 0.25, 32, 2, False),      # build operands, odd and even counts of them: a row's samples up to
+    (300, 260, 300e6, 1.5, 0.1, 32, 4, True),      # 16, 32 and 48
+    (301, 260, 300e6, 1.2, 0.1, 32, 4, False),
+    (420, 400, 300e6, 1.5, 0.25, 32, 6, True),
+    (400, 400, 300e6, 1.5, 0.25, 32, 6, False),
+    (300, 260, 300e6, 1.5, 0.15, 16, 4, True),
+    (300, 260, 300e6, 1.5, 0.1, 16, 4, False),
+])
+def test_final_stage_with_fewer_items_than_warps(oracle_lib, P, K, bw, ap, sp, T, items, odd):
+    """625 tiles of 32 x 32 pixels or 2,500 of 16 x 16, several units for every block, whose producer warps have items in
+    some subapertures only: against the float64 oracle (as above: below 1e-5), and the same bits twenty times."""
+    from fastsar_b200 import ImageFormer, sim
+    n = 800
+    col = sim.spotlight(P, K, 9.6e9, bw, 600e3, 45.0, ap)
+    rng = np.random.default_rng(P + K)
+    pos, amp = sim.scene(rng, n, n, sp, sp, n_points=12)
+    S = sim.add_noise(sim.simulate_brute(col, pos, amp), 0.01, rng).astype(np.complex64)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, n, n, sp, sp, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), T=T)
+    last = f._plan['levels'][-1]
+    groups = -(-last['Ko'] // 8)                   # of 8 samples: 64 / T to an item, A and B, 32 / T tiles to a unit
+    assert (32 // T) * 2 * -(-groups // (64 // T)) == items and last['Po'] % 2 == odd
+    form, _ = oracle_lib.image_former(col.ant, col.fmin, col.df, K, n, n, sp, sp, e1=(0.0, 1.0, 0.0),
+                                      e2=(1.0, 0.0, 0.0), T=T, kind='port')
+    dS = torch.from_numpy(S).cuda()
+    img = f.form_device(dS).clone()
+    e = _rel(img.cpu().numpy(), form(S))
+    print(f'{P} x {K} at T {T}: {items} items, rel {e:.2e}')
+    assert e < 1e-5
+    for _ in range(19):
+        assert torch.equal(torch.view_as_real(f.form_device(dS)), torch.view_as_real(img))
+
+
 def test_float32_form_with_large_phases_keeps_its_kernel(oracle_lib):
     """A level whose rotation phases pass the bound runs on the CUDA cores (its image is what it was), the later ones on
     the tensor cores; a non-finite sample is named by either."""
