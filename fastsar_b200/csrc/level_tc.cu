@@ -175,15 +175,20 @@ cudaError_t launch_fir(FirArgs f, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// The largest |component| of n floats of complex samples. 16-byte reads from the first 16-byte boundary on: a history is
+// aligned to its samples' 8 bytes (one of a stack of odd-sized histories lies between two boundaries).
 __global__ void amax_kernel(const float *__restrict__ v, size_t n, int *amax)
 {
     float m = 0.f;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(v) + i);
+    const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    const size_t head = ((uintptr_t)v & 15) && n >= 2 ? 2 : 0, n4 = (n - head) / 4;
+    const float4 *v4 = reinterpret_cast<const float4 *>(v + head);
+    for (size_t i = gid; i < n4; i += step) {
+        const float4 q = __ldg(v4 + i);
         m = fmaxf(m, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
     }
-    for (size_t i = (n / 4) * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(v[i]));
+    for (size_t i = head + n4 * 4 + gid; i < n; i += step) m = fmaxf(m, fabsf(v[i]));
+    if (gid < head) m = fmaxf(m, fabsf(v[gid]));
     if (!isfinite(m)) m = 0.f;                                 // non-finite samples are reported by the level kernel
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));

@@ -136,8 +136,8 @@ int ffbp_plan_destroy(ffbp_plan *plan);
 /* Bytes of device workspace a form call needs (the level intermediates and a status word).                     */
 int ffbp_plan_workspace_bytes(const ffbp_plan *plan, size_t *bytes);
 
-/* Form the image: d_S [P0, K0] complex64 phase history (unwindowed; the plan's window is applied here) ->
- * d_img [nx, ny] complex64. d_ws: the workspace (ffbp_plan_workspace_bytes, 256-byte aligned). The device the plan
+/* Form the image: d_S [P0, K0] complex64 phase history (unwindowed; the plan's window is applied here; aligned to 8
+ * bytes, as a complex64 array is) -> d_img [nx, ny] complex64. d_ws: the workspace (ffbp_plan_workspace_bytes, 256-byte aligned). The device the plan
  * was created on must be current (FFBP_E_ARG otherwise). Asynchronous on `stream`. The first non-finite sample's
  * pulse index (or -1) is written to h_bad_pulse when it is not NULL, which makes the call wait for the stream.
  * Failure reports of the tensor-core kernels: every bounded wait of theirs that runs out (a pipeline that stopped

@@ -100,6 +100,28 @@ def test_final_stage_with_fewer_items_than_warps(oracle_lib, P, K, bw, ap, sp, T
         assert torch.equal(torch.view_as_real(f.form_device(dS)), torch.view_as_real(img))
 
 
+@pytest.mark.parametrize('precision', ['float32', 'float16'])
+def test_history_between_16_byte_boundaries(precision):
+    """The second history of a stack of odd-sized ones starts 8 bytes past a 16-byte boundary: the bits of its copy's
+    image, also with the largest sample at the ends, which the scan reads apart (a scan that misses it scales by 256 too
+    much and reports the sample as non-finite)."""
+    from fastsar_b200 import ImageFormer, sim
+    P, K, n = 97, 83, 65
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), T=16,
+                    precision=precision)
+    gen = torch.Generator(device='cuda').manual_seed(1)
+    stack = torch.randn((2, P, K), dtype=torch.complex64, device='cuda', generator=gen)
+    assert stack[1].data_ptr() % 16 == 8
+    for at in (None, (0, 0), (0, 1), (P - 1, K - 1), (P - 1, K - 2)):
+        if at is not None:
+            stack[1][at] = 1e6
+        a = f.form_device(stack[1]).clone()
+        assert torch.equal(torch.view_as_real(a), torch.view_as_real(f.form_device(stack[1].clone())))
+        if at is not None:
+            stack[1][at] = 0.0
+
+
 def test_float32_form_with_large_phases_keeps_its_kernel(oracle_lib):
     """A level whose rotation phases pass the bound runs on the CUDA cores (its image is what it was), the later ones on
     the tensor cores; a non-finite sample is named by either."""
