@@ -18,6 +18,8 @@ KIND_NAMES = {1: 'amax', 2: 'level_fp32', 3: 'level_tc_gemm', 4: 'level_tc_fir',
               7: 'level_tc'}
 FFBP_KIND_LEVEL_TC_GEMM, FFBP_KIND_FINAL_TC, FFBP_KIND_LEVEL_TC = 3, 6, 7
 FFBP_LEVELS_TC2 = 0x200
+# flag (with FFBP_FINAL_FP32): the final stage on the CUDA cores whatever its shape
+FFBP_FINAL_CORES = 0x400
 
 # every symbol include/ffbp_b200.h declares
 EXPORTS = ('ffbp_last_error', 'ffbp_abi_version', 'ffbp_plan_create', 'ffbp_plan_destroy', 'ffbp_plan_workspace_bytes',

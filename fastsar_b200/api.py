@@ -15,8 +15,8 @@ Backends: 'auto' and 'cuda' run on the GPU. There is no CPU, JAX or TPU path in 
 ValueError, as the reference does for a backend its machine lacks.
 
 Precision: 'float32' (default): float32 arithmetic, or split float16 products (22 bits) accumulated in float32 on the
-tensor cores: the final stage (without an aperture weight) and the levels of small rotation phases. FASTSAR_FINAL=tc3
-takes the final stage in split bfloat16 (the reference's float32 CUDA default, fastsar/ffbp_cuda.py:949-953). 'float16': the final stage's operands in float16 on the tensor cores with
+tensor cores: the final stage (without an aperture weight) and the levels of small rotation phases. FASTSAR_FINAL=fp32
+keeps the final stage on the CUDA cores, FASTSAR_FINAL=tc3 takes it in split bfloat16 (the reference's float32 CUDA default, fastsar/ffbp_cuda.py:949-953). 'float16': the final stage's operands in float16 on the tensor cores with
 float32 accumulation (T = 16 or 32).
 """
 import ctypes
@@ -100,8 +100,8 @@ def _check_grid(nx, ny, spx, spy, e1, e2):
 
 
 def _final_mode(precision):
-    """The formation mode of a precision: 'float32' the float32 form (FASTSAR_FINAL=tc3 puts its final stage
-    in split bfloat16); 'float16' the levels and the final stage on the tensor cores, the levels in
+    """The formation mode of a precision: 'float32' the float32 form (FASTSAR_FINAL=fp32 keeps its final stage on the
+    CUDA cores, tc3 puts it in split bfloat16); 'float16' the levels and the final stage on the tensor cores, the levels in
     two passes through a float16 intermediate (FASTSAR_LEVELS=tc1: in one pass; fp32: on the float32 kernel)."""
     if precision == 'float16':
         lv = os.environ.get('FASTSAR_LEVELS', 'tc').strip().lower() or 'tc'
@@ -110,10 +110,11 @@ def _final_mode(precision):
         flags = {'tc': _lib.FFBP_LEVELS_TC | _lib.FFBP_LEVELS_TC2, 'tc1': _lib.FFBP_LEVELS_TC,
                  'tc2': _lib.FFBP_LEVELS_TC | _lib.FFBP_LEVELS_TC2, 'fp32': 0}[lv]
         return _lib.FFBP_FINAL_TC_F16 | flags
-    choice = os.environ.get('FASTSAR_FINAL', 'fp32').strip().lower() or 'fp32'
-    if choice not in ('fp32', 'tc3'):
+    choice = os.environ.get('FASTSAR_FINAL', '').strip().lower()
+    if choice not in ('', 'fp32', 'tc3'):
         raise ValueError(f"FASTSAR_FINAL must be 'fp32' or 'tc3', got {choice!r}")
-    return _lib.FFBP_FINAL_TC_BF16X3 if choice == 'tc3' else _lib.FFBP_FINAL_FP32
+    return {'': _lib.FFBP_FINAL_FP32, 'fp32': _lib.FFBP_FINAL_FP32 | _lib.FFBP_FINAL_CORES,
+            'tc3': _lib.FFBP_FINAL_TC_BF16X3}[choice]
 
 
 class DevicePlan:

@@ -235,9 +235,10 @@ double level_cycles(const ffbp_level_desc &L, int B, double kc)
 // cycles, 1.8e-5 at 195, 2.7e-5 at 317, 1.2e-4 at 1,870), and a plan's image is to stay what it was to 2e-5.
 constexpr double TC_F32_CYCLES = 170.0;
 
-// How each level runs, and the scratch of the two-pass ones. float32 form: two passes through a float32 intermediate
-// where the shape is covered and the phases are small. FFBP_LEVELS_TC: in one pass, or with FFBP_LEVELS_TC2 (and for shapes the one-pass kernel
-// does not cover) in two through a float16 intermediate; shapes that form does not cover stay in float32. A plan whose
+// How each level runs, and the scratch of the two-pass ones. float32 form (and split bfloat16 final stage): two passes
+// through a float32 intermediate where the shape is covered and the phases are small. FFBP_FINAL_TC_F16 with
+// FFBP_LEVELS_TC: in one pass, or with FFBP_LEVELS_TC2 (and for shapes the one-pass kernel does not cover) in two through
+// a float16 intermediate; shapes that form does not cover stay in float32; without it, on the CUDA cores. A plan whose
 // level outputs fit the static workspace keeps its scratch inside it too (ffbp_form_static).
 void plan_forms(ffbp_plan *p)
 {
@@ -259,7 +260,8 @@ void plan_forms(ffbp_plan *p)
     p->scratch = f16;
     for (auto &v : p->lv) {
         const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
-        if (!(p->final_mode & FFBP_LEVELS_TC) && !(v.cycles <= TC_F32_CYCLES)) continue;
+        if (!(p->final_mode & FFBP_LEVELS_TC) && ((p->final_mode & 0xff) == FFBP_FINAL_TC_F16 || !(v.cycles <= TC_F32_CYCLES)))
+            continue;
         if (v.form != LV_FP32 || (Lp + v.Dp - 1) / v.Dp > 16 || !two_pass_chunk(v, sizeof(float2), limit) ||
             !ffbp::level_mma_supported(v.C, Lk, v.Dk, v.nj))
             continue;
@@ -311,7 +313,8 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
     {
         const int fm = d->final_mode & 0xff, flags = d->final_mode & ~0xff;
         if ((fm != FFBP_FINAL_FP32 && fm != FFBP_FINAL_TC_F16 && fm != FFBP_FINAL_TC_BF16X3) ||
-            (flags & ~(FFBP_LEVELS_TC | FFBP_LEVELS_TC2)))
+            (flags & ~(FFBP_LEVELS_TC | FFBP_LEVELS_TC2 | FFBP_FINAL_CORES)) ||
+            ((flags & FFBP_FINAL_CORES) && fm != FFBP_FINAL_FP32))
             return fail(FFBP_E_ARG, "unknown final_mode %d", d->final_mode);
     }
     if (d->nlev > 8) return fail(FFBP_E_ARG, "%d levels, at most 8", d->nlev);
@@ -440,8 +443,8 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "final seeds kernel"));
     }
     // the float32 form: split float16 products on the tensor cores where they cover the shape; with aperture weights,
-    // which nothing bounds to float16's range, the CUDA cores
-    p->final_x2 = (d->final_mode & 0xff) == FFBP_FINAL_FP32 && !p->wf && ffbp::final_tc32_supported(p->T, B, p->Pf, p->Qf);
+    // which nothing bounds to float16's range, or where the caller asks for them, the CUDA cores
+    p->final_x2 = (d->final_mode & 0xff) == FFBP_FINAL_FP32 && !(d->final_mode & FFBP_FINAL_CORES) && !p->wf && ffbp::final_tc32_supported(p->T, B, p->Pf, p->Qf);
     if (p->final_x2) {
         if ((e = p->alloc(&p->seeds, 2 * (size_t)B * d->Pf)) != cudaSuccess) return cleanup(cuda_fail(e, "allocate final seeds"));
         e = ffbp::launch_final_seeds2(p->ux, p->uy, (long)B * d->Pf, p->spx, p->spy, p->a0, p->a1, p->seeds, s);

@@ -45,7 +45,8 @@ enum {
                             /* aperture weights) and its levels of small rotation phases run as split float16      */
                             /* products (22 bits, float32 sums) on the tensor cores, else on the CUDA cores;       */
                             /* ffbp_final takes the CUDA cores                                                     */
-    FFBP_FINAL_TC_F16 = 1,  /* tcgen05 tensor cores, float16 operands, float32 accumulation; ffbp_form scales  */
+    FFBP_FINAL_TC_F16 = 1,  /* tcgen05 tensor cores, float16 operands, float32 accumulation (the levels, without   */
+                            /* FFBP_LEVELS_TC, in float32 on the CUDA cores); ffbp_form scales                    */
                             /* the samples by a power of two into float16's range, ffbp_final takes them as    */
                             /* given (each component below 2^14 in magnitude)                                   */
     FFBP_FINAL_TC_BF16X3 = 2, /* tcgen05 tensor cores, operands split x = hi + lo in bfloat16, the hi*hi, hi*lo, */
@@ -57,9 +58,10 @@ enum {
                               /* the FIR's running sums in tensor memory. Levels the one-pass kernel does not   */
                               /* cover (more than 8 output pulses per input pulse) take the two-pass form below; */
                               /* levels of more than 64 children or 96 frequency taps keep a float32 intermediate */
-    FFBP_LEVELS_TC2 = 0x200   /* flag, with FFBP_LEVELS_TC: every tensor-core level in two passes (the product   */
+    FFBP_LEVELS_TC2 = 0x200,  /* flag, with FFBP_LEVELS_TC: every tensor-core level in two passes (the product   */
                               /* and ramp into a float16 intermediate in the workspace, then the pulse FIR in   */
                               /* float32), the form before the one-pass kernel                                    */
+    FFBP_FINAL_CORES = 0x400  /* flag, with FFBP_FINAL_FP32: the final stage on the CUDA cores whatever its shape */
 };
 
 /* Launch options of a tensor-core level (no counterpart in the reference, whose kernels take fixed shapes). 0 in a

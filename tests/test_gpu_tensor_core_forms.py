@@ -122,6 +122,30 @@ def test_history_between_16_byte_boundaries(precision):
             stack[1][at] = 0.0
 
 
+@pytest.mark.parametrize('name,value,precision,kinds,bound', [
+    ('FASTSAR_FINAL', 'fp32', 'float32', {'final_fp32'}, 1e-5),
+    ('FASTSAR_FINAL', 'tc3', 'float32', {'final_tc'}, 1e-4),          # split bfloat16: 16 bits
+    ('FASTSAR_LEVELS', 'fp32', 'float16', {'level_fp32', 'final_tc'}, 2e-3),    # a float16 final stage: 2^-11
+])
+def test_switches_choose_their_kernels(monkeypatch, name, value, precision, kinds, bound):
+    """FASTSAR_FINAL=fp32 keeps the float32 form's final stage on the CUDA cores and FASTSAR_LEVELS=fp32 all of the float16
+    form's levels, also where the tensor cores cover the shape: the kernels by name, and the default form's image."""
+    from fastsar_b200 import ImageFormer, sim
+    P, K, n = 128, 96, 64
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    args = (col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0))
+    S = torch.randn((P, K), dtype=torch.complex64, device='cuda', generator=torch.Generator(device='cuda').manual_seed(2))
+    out = torch.empty((n, n), dtype=torch.complex64, device='cuda')
+    monkeypatch.delenv('FASTSAR_FINAL', raising=False)
+    monkeypatch.delenv('FASTSAR_LEVELS', raising=False)
+    want = ImageFormer(*args, precision=precision).form_device(S).cpu().numpy()
+    monkeypatch.setenv(name, value)
+    f = ImageFormer(*args, precision=precision)
+    run = [k for k, _, _ in f._dev.form_profile(S, out)]
+    assert {k for k in run if k.startswith(name[8:13].lower())} | {run[-1]} == kinds, run
+    assert _rel(f.form_device(S).cpu().numpy(), want) < bound
+
+
 def test_float32_form_with_large_phases_keeps_its_kernel(oracle_lib):
     """A level whose rotation phases pass the bound runs on the CUDA cores (its image is what it was), the later ones on
     the tensor cores; a non-finite sample is named by either."""

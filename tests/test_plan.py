@@ -194,3 +194,22 @@ def test_packaged_level_options_cache_is_well_formed(tmp_path, monkeypatch):
     monkeypatch.setattr(tune, '_CACHE_LOADED', False)
     tune._load_cache()
     assert tune._LEVEL_CACHE[(1, 2, 3, 4, 5, 6, 7, 8, 9, 10)] == dict(nt=64, fir=2)
+
+
+def test_formation_mode_switches(monkeypatch):
+    """FASTSAR_FINAL and FASTSAR_LEVELS: what each value asks of a plan, and which are refused."""
+    from fastsar_b200 import _lib
+    from fastsar_b200.api import _final_mode
+    tc2 = _lib.FFBP_FINAL_TC_F16 | _lib.FFBP_LEVELS_TC | _lib.FFBP_LEVELS_TC2
+    for name, precision, modes in (
+            ('FASTSAR_FINAL', 'float32', {None: 0, '': 0, 'fp32': _lib.FFBP_FINAL_CORES, ' TC3 ': _lib.FFBP_FINAL_TC_BF16X3}),
+            ('FASTSAR_LEVELS', 'float16', {None: tc2, '': tc2, 'tc2': tc2, 'tc1': _lib.FFBP_FINAL_TC_F16 | _lib.FFBP_LEVELS_TC,
+                                           'fp32': _lib.FFBP_FINAL_TC_F16})):
+        for value, mode in modes.items():
+            monkeypatch.delenv(name, raising=False)
+            if value is not None:
+                monkeypatch.setenv(name, value)
+            assert _final_mode(precision) == mode, (name, value)
+        monkeypatch.setenv(name, 'fp64')
+        with pytest.raises(ValueError, match=name):
+            _final_mode(precision)
