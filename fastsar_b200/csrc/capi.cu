@@ -126,6 +126,7 @@ struct ffbp_plan {
     float *wp = nullptr, *wk = nullptr, *wf = nullptr;
     double *ux = nullptr, *uy = nullptr, *ucx = nullptr, *ucy = nullptr, *rc = nullptr;
     float4 *seeds = nullptr;          // the tensor-core final stage's ramp seeds [ntiles, Pf], two each in split float16
+    int wexp = 0;                     // the window's power of two (window_exponent)
     bool final_x2 = false;            // the float32 form's final stage in split float16 on the tensor cores
     int2 *first = nullptr;
     size_t bufA = 0, bufB = 0;
@@ -234,6 +235,22 @@ double level_cycles(const ffbp_level_desc &L, int B, double kc)
 // does not make; past about 170 cycles (rms 110) the two differ by more than 1.5e-5 of the image (measured: 9e-6 at 160
 // cycles, 1.8e-5 at 195, 2.7e-5 at 317, 1.2e-4 at 1,870), and a plan's image is to stay what it was to 2e-5.
 constexpr double TC_F32_CYCLES = 170.0;
+
+// The power of two of the window's largest product where that is far from one (LevelLaunch::wexp): the first level's scale
+// comes from the history's largest sample before the window, and leaves float16's range room for a few powers of two only.
+// Ordinary windows (a Taylor window of sum P: 2.8) are left as they are.
+int window_exponent(const float *wp, int P, const float *wk, int K)
+{
+    auto most = [](const float *w, int n) {
+        double m = 0.0;
+        for (int i = 0; w && i < n; ++i) m = std::max(m, std::fabs((double)w[i]));
+        return w ? m : 1.0;
+    };
+    const double m = wp ? most(wp, P) * most(wk, K) : 1.0;
+    int ex = 0;
+    if (m > 0.0 && std::isfinite(m) && (m > 4.0 || m < 0.25)) std::frexp(m, &ex);
+    return ex;
+}
 
 // How each level runs, and the scratch of the two-pass ones. float32 form (and split bfloat16 final stage): two passes
 // through a float32 intermediate where the shape is covered and the phases are small. FFBP_FINAL_TC_F16 with
@@ -412,6 +429,7 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
     if (d->partial ? (long)B * d->T * d->T > (long)d->Nx * d->Ny : (long)B * d->T * d->T != (long)d->Nx * d->Ny)
         return cleanup(fail(FFBP_E_ARG, "tiles %d of %d^2 do not %s %dx%d", B, d->T, d->partial ? "fit" : "cover", d->Nx, d->Ny));
     void *q;
+    p->wexp = window_exponent(d->h_wp, d->levels[0].P, d->h_wk, d->levels[0].K);
     if (d->h_wp) {
         if ((e = upload(d->h_wp, sizeof(float) * d->levels[0].P, &q, true)) != cudaSuccess) return cleanup(cuda_fail(e, "upload window"));
         p->wp = (float *)q;
@@ -527,6 +545,7 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
         L.Np = v.Np; L.C = v.C; L.P = v.P; L.K = v.K; L.Ko = v.Ko; L.Po = v.Po; L.Dk = v.Dk; L.Lk = v.Lk; L.plk = v.plk;
         L.Dp = v.Dp; L.Lp = v.Lp; L.plp = v.plp; L.kc = v.kc;
         L.amax = amax + l + 1;
+        L.wexp = l == 0 ? p->wexp : 0;
         L.test_wait_ns = p->test_kind == FFBP_KIND_LEVEL_TC ? p->test_ns : 0u;
         L.tc_nt = v.tc.nt; L.tc_sb = v.tc.sb; L.tc_pc = v.tc.copies; L.tc_rp = v.tc.repeat; L.tc_fir = v.tc.fir;
         L.tc_cw = v.tc.consumers;

@@ -35,6 +35,19 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// e of the power of two 2^e that a tensor-core level's intermediate is scaled by: values up to 4 m (m the input's largest
+// component; the taps' absolute sum is below 4 for the decimators of any plan) come below 2^13, times the window's 2^wexp
+// (LevelLaunch::wexp): a float16 intermediate then stays in range and keeps 11 significant bits. 2^e, 2^-e and an eighth of
+// either are normal float32 numbers.
+__device__ __forceinline__ int level_exponent(const int *amax, int wexp)
+{
+    const float m = amax ? __int_as_float(*amax) : 0.f;
+    if (!(m > 0.f) || !isfinite(m)) return 0;
+    int ex;
+    frexpf(m, &ex);                                             // m < 2^ex
+    return min(max(11 - ex - wexp, -120), 120);
+}
+
 // Two float32 fused multiply-adds in one instruction (sm_100's packed FMA): (a.x b.x + c.x, a.y b.y + c.y), each
 // rounded as fmaf rounds it.
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)

@@ -207,8 +207,7 @@ __device__ __forceinline__ float operand_scale(const int *amax)
     if (!(m > 0.f) || !isfinite(m)) return 1.f;
     int ex;
     frexpf(m, &ex);                                             // m < 2^ex
-    ex = ex < -100 ? -100 : (ex > 100 ? 100 : ex);
-    return ldexpf(1.f, 13 - ex);
+    return ldexpf(1.f, min(max(13 - ex, -120), 120));           // it and its inverse normal float32 numbers
 }
 
 // The operands' arithmetic: float16, or x = hi + lo in bfloat16 (16 bits) or in float16 (22 bits).

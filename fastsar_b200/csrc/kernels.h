@@ -18,6 +18,8 @@ struct LevelLaunch {
     int Np, C, P, K, Ko, Po, Dk, Lk, plk, Dp, Lp, plp;
     double kc;
     int *amax = nullptr;  // or the largest |component| of the output, as float bits (atomicMax; start at 0)
+    int wexp = 0;         // tensor-core levels: the power of two of the window's largest product |wp wk| where it is above 4
+                          // or below 1/4, by which a windowed sample's scale is reduced; 0 for ordinary windows
     unsigned test_wait_ns = 0;   // tensor-core pass 1 only, for tests of the failure report: when nonzero the MMA
                                  // issuer first waits this long on a barrier nothing completes, as a stuck pipeline
     // tensor-core pass 1 launch options (0: the default): output columns per tile, B stages, plane copies (2 or 4),

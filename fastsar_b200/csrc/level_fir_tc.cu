@@ -45,28 +45,18 @@ constexpr int MO = 128;                        // output pulses per tile
 constexpr uint64_t R_WAIT_NS = 2000000000ull;
 
 struct FirTcArgs {
-    const __half2 *__restrict__ y;    // [rows, P, Kop], scaled by y_scale(amax_in)
+    const __half2 *__restrict__ y;    // [rows, P, Kop], times 2^level_exponent
     const float *__restrict__ tp;     // [Lp] (null: Dp = 1, one tap 1)
     float2 *out;                      // [rows, Po, Ko]
     int *amax;                        // largest |component| of the output (float bits) or null
     const int *amax_in;
+    int wexp;
     int *err;
     int rows, P, Kop, Ko, Po, Dp, Lp, plp;
     int NC, ncb, nob;                 // complex columns per tile, column tiles, output-pulse tiles
     long ntiles;
     int NQ;                           // 16-byte words per shifted tap copy
 };
-
-// The power of two the first pass scaled the intermediate by (level_tc_gemm's y_scale).
-__device__ __forceinline__ float fir_inv_scale(const int *amax)
-{
-    const float m = amax ? __int_as_float(*amax) : 0.f;
-    if (!(m > 0.f) || !isfinite(m)) return 1.f;
-    int ex;
-    frexpf(4.f * m, &ex);
-    ex = ex < -100 ? -100 : (ex > 100 ? 100 : ex);
-    return ldexpf(1.f, ex - 13);
-}
 
 struct TileGeom {
     int row, i0, mo, j0;              // row; first output pulse and count; first column
@@ -270,7 +260,7 @@ __global__ void __launch_bounds__(R_NTHR, 1) level_fir_tc_kernel(const FirTcArgs
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (warps 0..3)
-        const float inv = fir_inv_scale(a.amax_in);
+        const float inv = ldexpf(1.f, -level_exponent(a.amax_in, a.wexp));
         float vmax = 0.f;
         long t_it = 0;
         for (long ti = blockIdx.x; ti < a.ntiles; ti += gridDim.x, ++t_it) {
@@ -368,7 +358,7 @@ cudaError_t launch_level_fir_tc(const LevelLaunch &L, const int *amax_in, const 
 {
     *why = nullptr;
     FirTcArgs a;
-    a.y = static_cast<const __half2 *>(scratch); a.out = L.out; a.amax = L.amax; a.amax_in = amax_in; a.err = err;
+    a.y = static_cast<const __half2 *>(scratch); a.out = L.out; a.amax = L.amax; a.amax_in = amax_in; a.wexp = L.wexp; a.err = err;
     a.rows = L.Np * L.C; a.P = L.P; a.Kop = (L.Ko + 3) & ~3; a.Ko = L.Ko; a.Po = L.Po; a.Dp = L.Dp;
     a.Lp = L.Dp > 1 ? L.Lp : 1; a.plp = L.Dp > 1 ? L.plp : 0; a.tp = L.Dp > 1 ? L.tp : nullptr;
     a.ncb = (a.Kop + 127) / 128;

@@ -56,7 +56,7 @@ constexpr int M_PHB = 3;                     // ring of phase batches
 constexpr int M_ND = 4;                      // most accumulator buffers
 constexpr int M_NBAR = 2 * 4 + 2 * 4 + 2 * M_ND + 2 * M_PHB + 2;   // barriers
 constexpr uint64_t M_WAIT_NS = 2000000000ull;
-constexpr float M_TAP_SCALE = 8.f;           // the taps' power of two; the samples' is y_scale / M_TAP_SCALE
+constexpr float M_TAP_SCALE = 8.f;           // the taps' power of two; the samples' is 2^level_exponent / M_TAP_SCALE
 
 struct MmaArgs {
     const float2 *__restrict__ x;     // [Np, P, K]
@@ -66,7 +66,8 @@ struct MmaArgs {
     const float *__restrict__ wk;     // [K] or null
     int *bad;                         // first non-finite pulse or null
     const int *amax_in;
-    void *y;                          // [nn, C, P, Kop] from parent n0, column j0: half2 or float2, times y_scale
+    int wexp;                         // the window's power of two (LevelLaunch::wexp)
+    void *y;                          // [nn, C, P, Kop] from parent n0, column j0: half2 or float2, times 2^level_exponent
     int *err;
     int n0, C, P, K, Dk, Lk, plk;
     int j0, nj, Kop;                  // the first column, the columns and their pitch in y
@@ -124,7 +125,7 @@ __device__ __forceinline__ void split8(const float *v, uint4 &hi, uint4 &lo)
 }
 
 // Bits 15 and 31 set where one of 8 float16 values is not finite (its exponent all ones carries into the sign's place): a
-// sample scaled below 2^8 is finite in float16 unless it was not in float32.
+// finite sample is scaled below 2^8, its product with the window below 2^10 (LevelLaunch::wexp), finite in float16.
 __device__ __forceinline__ uint32_t non_finite(uint4 v)
 {
     auto c = [](uint32_t x) { return (x & 0x7c007c00u) + 0x04000400u; };
@@ -144,17 +145,6 @@ __device__ __forceinline__ float2 cis_accurate(float u, float r)
     float s, c;
     sincospif(2.f * ((m - rintf(m)) + fmaf(u, r, -m)), &s, &c);
     return make_float2(c, s);
-}
-
-// The samples' power of two: y_scale (level_tc.cu) less the taps'.
-__device__ __forceinline__ float sample_scale(const int *amax)
-{
-    const float m = amax ? __int_as_float(*amax) : 0.f;
-    if (!(m > 0.f) || !isfinite(m)) return 1.f / M_TAP_SCALE;
-    int ex;
-    frexpf(4.f * m, &ex);
-    ex = ex < -100 ? -100 : (ex > 100 ? 100 : ex);
-    return ldexpf(1.f / M_TAP_SCALE, 13 - ex);
 }
 
 __device__ __forceinline__ bool elect_one()
@@ -242,7 +232,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
         sH[i] = in ? (a.tk ? a.tk[r] : 1.f) * M_TAP_SCALE : 0.f;
     }
     // the samples' power of two, which the window's table carries too (exact)
-    const float xs = sample_scale(a.amax_in);
+    const float xs = ldexpf(1.f / M_TAP_SCALE, level_exponent(a.amax_in, a.wexp));
     if (WIN && a.wtab)
         for (int i = t; i < a.K; i += M_NTHR) sW[i] = (a.wk ? a.wk[i] : 1.f) * xs;
     if (warp == M_MW) {
@@ -792,7 +782,7 @@ cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, 
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     MmaArgs a;
     a.x = L.x; a.ph = L.phase; a.tk = L.Dk > 1 ? L.tk : nullptr; a.wp = L.wp; a.wk = L.wk; a.bad = L.bad;
-    a.amax_in = amax_in; a.y = y; a.err = err; a.wtab = tab; a.n0 = n0; a.C = L.C; a.P = L.P; a.K = L.K; a.Dk = L.Dk; a.Lk = Lk;
+    a.amax_in = amax_in; a.wexp = L.wexp; a.y = y; a.err = err; a.wtab = tab; a.n0 = n0; a.C = L.C; a.P = L.P; a.K = L.K; a.Dk = L.Dk; a.Lk = Lk;
     a.plk = plk; a.j0 = j0; a.nj = nj; a.Kop = (nj + 3) & ~3; a.G = m.G; a.Gf = m.Gf; a.A = m.A; a.A8 = (m.A + 7) / 8; a.ks = m.ks; a.Ch = m.Ch;
     a.ncg = (L.C + m.Ch - 1) / m.Ch; a.TM = m.TM; a.ntile = (nj + m.TM * m.S - 1) / (m.TM * m.S);
     a.ROWS = m.ROWS; a.W = m.W; a.NT = m.NT; a.ZS = m.ZS; a.XR = m.XR; a.ntw = m.ntw; a.TW = m.NT > 2 ? 1 : m.ntw;

@@ -3,7 +3,7 @@
 //
 // Pass 1 (level_mma.cu): per parent and pulse the rotation and the frequency FIR of every child as one product on the
 // tensor cores, written at the input pulse rate as the intermediate y [Np, C, P, Kop]: float16 in the mixed-precision
-// form, float32 in the float32 form, times a power of two (y_scale).
+// form, float32 in the float32 form, times a power of two (2^level_exponent).
 //
 // Pass 2: the pulse FIR of the intermediate, written as complex64 with the largest component recorded: on the CUDA
 // cores in float32 (level_fir here: a thread per two columns with the ceil(Lp / Dp) outputs it feeds in registers), or
@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "common.cuh"
@@ -21,25 +22,14 @@ namespace ffbp {
 
 namespace {
 
-// The power of two that brings values up to 4 amax (the taps' absolute sum is below 4 for the decimators of any
-// plan) below 2^13: the float16 intermediate then stays in range and keeps 11 significant bits.
-__device__ __forceinline__ float y_scale(const int *amax)
-{
-    const float m = amax ? __int_as_float(*amax) : 0.f;
-    if (!(m > 0.f) || !isfinite(m)) return 1.f;
-    int ex;
-    frexpf(4.f * m, &ex);
-    ex = ex < -100 ? -100 : (ex > 100 ? 100 : ex);
-    return ldexpf(1.f, 13 - ex);
-}
-
 // --------------------------------------------------------------------------------------------------- pass 2
 struct FirArgs {
-    const void *__restrict__ y;       // [rows, P, Kop] float16 or float32 complex, times y_scale
+    const void *__restrict__ y;       // [rows, P, Kop] float16 or float32 complex, times 2^level_exponent
     const float *__restrict__ tp;     // [Lp]
     float2 *__restrict__ out;         // [rows, Po, Ko], columns nj of it from this pointer on
     int *amax;
     const int *amax_in;
+    int wexp;
     int rows, P, Kop, nj, Ko, Po, Dp, Lp, plp, SEG, nseg;
 };
 
@@ -81,7 +71,7 @@ __global__ void __launch_bounds__(128) level_fir(const FirArgs a)
     if (gid >= (long)a.rows * npair) return;
     const int row = (int)(gid / npair), j = 2 * (int)(gid - (long)row * npair);
     const int seg = blockIdx.y;
-    const float inv = 1.f / y_scale(a.amax_in);
+    const float inv = ldexpf(1.f, -level_exponent(a.amax_in, a.wexp));
     const int i_s = seg * a.SEG, i_e = min(a.Po, i_s + a.SEG);
     const int g_end = i_e + AP - 1;
     const PT *__restrict__ yr = static_cast<const PT *>(a.y) + ((size_t)row * a.P * a.Kop + j) / 2;   // Kop, j even
@@ -175,21 +165,33 @@ cudaError_t launch_fir(FirArgs f, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// The largest |component| of n floats of complex samples. 16-byte reads from the first 16-byte boundary on: a history is
-// aligned to its samples' 8 bytes (one of a stack of odd-sized histories lies between two boundaries).
+// The largest |component| of n floats of complex samples, the non-finite ones left out (the level's kernel reports them).
+// 16-byte reads from the first 16-byte boundary on: a history is aligned to its samples' 8 bytes (one of a stack of
+// odd-sized histories lies between two boundaries).
 __global__ void amax_kernel(const float *__restrict__ v, size_t n, int *amax)
 {
     float m = 0.f;
+    auto take = [&](float a) {
+        a = fabsf(a);
+        if (a <= FLT_MAX) m = fmaxf(m, a);
+    };
     const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     const size_t head = ((uintptr_t)v & 15) && n >= 2 ? 2 : 0, n4 = (n - head) / 4;
     const float4 *v4 = reinterpret_cast<const float4 *>(v + head);
     for (size_t i = gid; i < n4; i += step) {
         const float4 q = __ldg(v4 + i);
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
+        const float most = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w)));   // fmaxf passes NaNs over
+        if (most <= FLT_MAX) {
+            m = fmaxf(m, most);
+        } else {
+            take(q.x);
+            take(q.y);
+            take(q.z);
+            take(q.w);
+        }
     }
-    for (size_t i = head + n4 * 4 + gid; i < n; i += step) m = fmaxf(m, fabsf(v[i]));
-    if (gid < head) m = fmaxf(m, fabsf(v[gid]));
-    if (!isfinite(m)) m = 0.f;                                 // non-finite samples are reported by the level kernel
+    for (size_t i = head + n4 * 4 + gid; i < n; i += step) take(v[i]);
+    if (gid < head) take(v[gid]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(amax, __float_as_int(m));
@@ -296,7 +298,7 @@ static cudaError_t run_fir(const FirArgs &f, cudaStream_t s, const char **why)
 static FirArgs fir_args(const LevelLaunch &L, const int *amax_in, const void *scratch)
 {
     FirArgs f;
-    f.y = scratch; f.tp = L.Dp > 1 ? L.tp : nullptr; f.out = L.out; f.amax = L.amax; f.amax_in = amax_in;
+    f.y = scratch; f.tp = L.Dp > 1 ? L.tp : nullptr; f.out = L.out; f.amax = L.amax; f.amax_in = amax_in; f.wexp = L.wexp;
     f.rows = L.Np * L.C; f.P = L.P; f.Kop = (L.Ko + 3) & ~3; f.nj = f.Ko = L.Ko; f.Po = L.Po; f.Dp = L.Dp;
     f.Lp = L.Dp > 1 ? L.Lp : 1; f.plp = L.Dp > 1 ? L.plp : 0;
     return f;

@@ -249,7 +249,8 @@ int ffbp_level(const void *d_x, int Np, int P, int K, const void *d_phase, int C
  * modulated frequency taps tk[r] exp(2 pi i sl r) times the windows of the parent's row, operands split into float16
  * hi + lo, three products accumulated in float32; the ramp exp(2 pi i (c0 + sl (Dk j - plk - kc))); a float16 intermediate in d_scratch
  * (ffbp_level_tc_scratch_bytes, 16-byte aligned), scaled by a power of two from the input's largest component;
- * the pulse FIR in float32. C <= 64 and Lk <= 96 (FFBP_E_UNSUPPORTED otherwise). d_status: 3 ints, zeroed by the
+ * the pulse FIR in float32. C <= 64 and Lk <= 96 (FFBP_E_UNSUPPORTED otherwise); a window's products wp wk are to be
+ * of order one (a plan's may be of any size: its scale is taken at creation). d_status: 3 ints, zeroed by the
  * caller: [0] nonzero when a bounded wait of the kernel ran out, [1] the input's largest |component| (float bits,
  * filled here), [2] the output's. No counterpart in the reference (its levels run in float32 only).            */
 size_t ffbp_level_tc_scratch_bytes(int Np, int C, int P, int Ko);

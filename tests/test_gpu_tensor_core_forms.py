@@ -122,6 +122,53 @@ def test_history_between_16_byte_boundaries(precision):
             stack[1][at] = 0.0
 
 
+@pytest.mark.parametrize('precision', ['float32', 'float16'])
+@pytest.mark.parametrize('pulses,samples,amplitude', [
+    (1 / 4096.0, 1 / 2048.0, 1.0),    # a window normalised to a sum of one: products of 2^-23
+    (2.0 ** 12, 1.0, 1.0),            # products past float16's range
+    (1.0, 1.0, 2.0 ** 108),           # histories near either end of float32's range
+    # (at the lower end t = 2^-126 / 2^-112 of a sample, a level's output a tenth of it: flushed values below 10 t, of
+    # which there are 0.8 10 t, cost sqrt(0.27 (10 t)^3) = 8e-6 a level in any float32 kernel; at 2^-104 2e-9)
+    (1.0, 1.0, 2.0 ** -104),
+])
+def test_scales_of_window_and_history(precision, pulses, samples, amplitude):
+    """The image of a scaled window or history is the scaled image: powers of two, so that nothing but the split products'
+    place in float16's range can differ (2^-22 to 2^-24 a factor: below 2e-6, in the float16 form a rounding of the
+    intermediate here and there, 2^-12 each: below 5e-4), and nothing is taken for non-finite."""
+    from fastsar_b200 import ImageFormer, sim
+    from fastsar_b200.api import DevicePlan, _final_mode
+    P, K, n = 128, 96, 64
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), precision=precision)
+    S = torch.randn((P, K), dtype=torch.complex64, device='cuda', generator=torch.Generator(device='cuda').manual_seed(3))
+    out = torch.empty((n, n), dtype=torch.complex64, device='cuda')
+    want = f.form_device(S).cpu().numpy().astype(complex)
+    dev = DevicePlan(f._plan, (f.wp * np.float32(pulses)), (f.wk * np.float32(samples)), None, None, _final_mode(precision))
+    dev.form(S * amplitude, out)
+    got = out.cpu().numpy().astype(complex) / (pulses * samples * amplitude)
+    e = _rel(got, want)
+    print(f'{precision}: window {pulses * samples:.1e}, history {amplitude:.1e}: rel {e:.1e}')
+    assert e < (2e-6 if precision == 'float32' else 5e-4)
+
+
+def test_pulse_of_a_non_finite_sample_among_large_ones():
+    """An infinite or undefined sample names its pulse and no other, whatever the finite samples near it."""
+    from fastsar_b200 import ImageFormer, sim
+    P, K, n = 128, 96, 64
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0))
+    for bad in (float('inf'), float('nan')):
+        S = torch.ones((P, K), dtype=torch.complex64, device='cuda')
+        S[40, 50] = 1e9                                       # read by the same thread as the next sample
+        S[70, 51] = bad
+        S[40, 51] = bad
+        with pytest.raises(ValueError, match='pulse 40'):
+            f.form_device(S)
+        S[40, 51] = 0.0
+        with pytest.raises(ValueError, match='pulse 70'):
+            f.form_device(S)
+
+
 @pytest.mark.parametrize('name,value,precision,kinds,bound', [
     ('FASTSAR_FINAL', 'fp32', 'float32', {'final_fp32'}, 1e-5),
     ('FASTSAR_FINAL', 'tc3', 'float32', {'final_tc'}, 1e-4),          # split bfloat16: 16 bits
