@@ -41,23 +41,26 @@ int cuda_fail(cudaError_t e, const char *what)
     return fail(FFBP_E_CUDA, "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
 }
 
+// A level on the float32 CUDA-core kernel, on the one-pass tensor-core kernel, or in two passes through an intermediate
+// of float16 (the mixed-precision form) or float32 (the float32 form).
+enum LevelForm { LV_FP32 = 0, LV_ONE_PASS = 1, LV_TWO_PASS_F16 = 2, LV_TWO_PASS_F32 = 3 };
+
+// A level's form and, in two passes, what one launch pair takes: so many parents, children (all, or of one parent) and
+// output columns (all, or of one parent), whose intermediate fits the workspace's scratch.
+struct LevelRun { int form = LV_FP32, nn = 0, nc = 0, nj = 0; };
+
+inline bool two_pass(const LevelRun &r) { return r.form == LV_TWO_PASS_F16 || r.form == LV_TWO_PASS_F32; }
+
 struct DevLevel {
     int C, Dk, Dp, K, P, Ko, Po, Lk, plk, Lp, plp, Np;
     ffbp_tc_opts tc{};
     float *tk = nullptr, *tp = nullptr;
     float2 *phase = nullptr;
     double kc;
-    // how the level runs (plan_forms): LevelForm, and for the two-pass forms the parents and the output columns of one
-    // launch pair (its intermediate fits the workspace's scratch)
-    int form = 0, nn = 0, nj = 0;
+    // how the level runs (plan_forms): on the plan's whole workspace, and on the least one (ffbp_form_static)
+    LevelRun run, least;
     double cycles = 0.0;              // the largest rotation phase (cycles at the band's edge; level_cycles)
 };
-
-// A level on the float32 CUDA-core kernel, on the one-pass tensor-core kernel, or in two passes through an intermediate
-// of float16 (the mixed-precision form) or float32 (the float32 form).
-enum LevelForm { LV_FP32 = 0, LV_ONE_PASS = 1, LV_TWO_PASS_F16 = 2, LV_TWO_PASS_F32 = 3 };
-
-inline bool two_pass(const DevLevel &v) { return v.form == LV_TWO_PASS_F16 || v.form == LV_TWO_PASS_F32; }
 
 size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
@@ -130,7 +133,7 @@ struct ffbp_plan {
     bool final_x2 = false;            // the float32 form's final stage in split float16 on the tensor cores
     int2 *first = nullptr;
     size_t bufA = 0, bufB = 0;
-    size_t scratch = 0;               // bytes of the two-pass levels' intermediate
+    size_t scratch = 0, least_scratch = 0;   // bytes of the two-pass levels' intermediate (DevLevel::run, ::least)
     std::vector<void *> owned;
     // the host-memory pipeline of ffbp_form_host, made at its first call: an upload and a download stream, per
     // device buffer pair b the events "history b uploaded", "image b formed", "image b downloaded", and a pinned
@@ -189,25 +192,42 @@ struct ffbp_plan {
 namespace {
 
 // The largest intermediate of a two-pass level that the float32 form keeps at once: larger levels run in several launch
-// pairs (parents, or columns of one parent), so that a plan needs little more workspace than its level outputs.
+// pairs, so that a plan needs little more workspace than its level outputs. Smaller pieces were slower, L2 or not: 4,096 x
+// 4,096 samples to 2,048 x 2,048 pixels, first level 622 us whole (504 MiB), 840 in two of 256 MiB, 986 in four of 128;
+// 12,288 x 8,832 pixels, third level 15.7 ms in pieces of 2 GiB, 17.1 / 18.3 / 20.5 in 512 / 256 / 128 MiB.
 constexpr size_t Y_BYTES = size_t(2) << 30;
 
-// The parents and columns of one launch pair whose intermediate (es bytes a sample) fits `limit`; false when 128 columns
-// of one parent do not.
-bool two_pass_chunk(DevLevel &v, size_t es, size_t limit)
+size_t f32_scratch(const LevelRun &r, int P) { return (size_t)r.nn * r.nc * P * ((r.nj + 3) & ~3) * sizeof(float2); }
+
+// The launch pairs of a level in two passes whose float32 intermediate fits `limit`: as many parents as fit, else columns
+// of one parent by whole tiles of 128 (a pulse's taps are built once for a launch's columns), else 8 or more of its children
+// and 128 columns or more (its samples are converted once for a launch's children). false when 8 children's 128 columns
+// do not fit.
+bool two_pass_chunk(LevelRun &r, int Np, int C, int P, int Ko, size_t limit)
 {
-    const size_t col = (size_t)v.C * v.P * es, par = col * ((v.Ko + 3) & ~3);
+    const size_t one = (size_t)P * sizeof(float2), col = one * C, par = col * ((Ko + 3) & ~3);
+    auto columns = [&](int nc, int most) {
+        const int n = (Ko + most - 1) / most;
+        r.nn = 1;
+        r.nc = nc;
+        r.nj = std::min(Ko, ((Ko + n - 1) / n + 127) & ~127);
+    };
     if (par <= limit) {
-        const int most = (int)std::min<size_t>(limit / par, (size_t)v.Np), n = (v.Np + most - 1) / most;
-        v.nn = (v.Np + n - 1) / n;
-        v.nj = v.Ko;
+        const int most = (int)std::min<size_t>(limit / par, (size_t)Np), n = (Np + most - 1) / most;
+        r.nn = (Np + n - 1) / n;
+        r.nc = C;
+        r.nj = Ko;
         return true;
     }
-    const int most = (int)(limit / col) & ~127;
-    if (most < 128) return false;
-    const int n = (v.Ko + most - 1) / most;
-    v.nn = 1;
-    v.nj = std::min(most, ((v.Ko + n - 1) / n + 127) & ~127);
+    if (limit / col >= 128) {
+        columns(C, (int)std::min<size_t>(limit / col, 1 << 30) & ~127);
+        return true;
+    }
+    const size_t tile = one * ((std::min(Ko, 128) + 3) & ~3);                  // a child's 128 columns
+    const int most = (int)std::min<size_t>(limit / tile, 1 << 30) & ~7;
+    if (most < 8) return false;
+    const int n = (C + most - 1) / most, nc = std::min(C, ((C + n - 1) / n + 7) & ~7);
+    columns(nc, Ko <= 128 ? Ko : (int)std::min<size_t>(limit / (one * nc), 1 << 30) & ~127);
     return true;
 }
 
@@ -255,36 +275,45 @@ int window_exponent(const float *wp, int P, const float *wk, int K)
 // How each level runs, and the scratch of the two-pass ones. float32 form (and split bfloat16 final stage): two passes
 // through a float32 intermediate where the shape is covered and the phases are small. FFBP_FINAL_TC_F16 with
 // FFBP_LEVELS_TC: in one pass, or with FFBP_LEVELS_TC2 (and for shapes the one-pass kernel does not cover) in two through
-// a float16 intermediate; shapes that form does not cover stay in float32; without it, on the CUDA cores. A plan whose
-// level outputs fit the static workspace keeps its scratch inside it too (ffbp_form_static).
+// a float16 intermediate; shapes that form does not cover stay in float32; without it, on the CUDA cores. The least
+// workspace of a plan whose level outputs fit the static workspace fits there too (ffbp_form_static): its float32
+// intermediates take what the outputs leave, in as many launch pairs as that needs. (ffbp_form is not held to that: 1,024 x
+// 1,024 pixels, outputs of 33 MiB and a first intermediate of 132, form in 768 us with it whole, their first level 314.)
 void plan_forms(ffbp_plan *p)
 {
     const size_t base = 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2));
     size_t f16 = 0;
     for (auto &v : p->lv) {
         const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
-        v.form = LV_FP32;
         if (!(p->final_mode & FFBP_LEVELS_TC)) continue;
-        if (!(p->final_mode & FFBP_LEVELS_TC2) && ffbp::level_fused_supported(v.C, Lk, v.Dk, Lp, v.Dp)) v.form = LV_ONE_PASS;
+        if (!(p->final_mode & FFBP_LEVELS_TC2) && ffbp::level_fused_supported(v.C, Lk, v.Dk, Lp, v.Dp)) v.run.form = LV_ONE_PASS;
         else if (ffbp::level_tc_supported(v.C, Lk, v.Dk)) {
-            v.form = LV_TWO_PASS_F16;
-            v.nn = v.Np;
-            v.nj = v.Ko;
+            v.run = {LV_TWO_PASS_F16, v.Np, v.C, v.Ko};
             f16 = std::max(f16, ffbp::level_tc_scratch_bytes(v.Np, v.C, v.P, v.Ko));
         }
+        v.least = v.run;
     }
-    const size_t limit = base + align256(f16) <= FFBP_STATIC_WS_BYTES ? FFBP_STATIC_WS_BYTES - base : std::max(f16, Y_BYTES);
-    p->scratch = f16;
-    for (auto &v : p->lv) {
-        const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
-        if (!(p->final_mode & FFBP_LEVELS_TC) && ((p->final_mode & 0xff) == FFBP_FINAL_TC_F16 || !(v.cycles <= TC_F32_CYCLES)))
-            continue;
-        if (v.form != LV_FP32 || (Lp + v.Dp - 1) / v.Dp > 16 || !two_pass_chunk(v, sizeof(float2), limit) ||
-            !ffbp::level_mma_supported(v.C, Lk, v.Dk, v.nj))
-            continue;
-        v.form = LV_TWO_PASS_F32;
-        p->scratch = std::max(p->scratch, (size_t)v.nn * v.C * v.P * ((v.nj + 3) & ~3) * sizeof(float2));
-    }
+    auto float32_levels = [&](LevelRun DevLevel::*run, size_t limit) {
+        size_t scratch = f16;
+        for (auto &v : p->lv) {
+            const int Lk = v.Dk > 1 ? v.Lk : 1, Lp = v.Dp > 1 ? v.Lp : 1;
+            if (!(p->final_mode & FFBP_LEVELS_TC) && ((p->final_mode & 0xff) == FFBP_FINAL_TC_F16 || !(v.cycles <= TC_F32_CYCLES)))
+                continue;
+            LevelRun r;
+            if ((v.*run).form != LV_FP32 || (Lp + v.Dp - 1) / v.Dp > 16 || !two_pass_chunk(r, v.Np, v.C, v.P, v.Ko, limit) ||
+                !ffbp::level_mma_supported(r.nc, Lk, v.Dk, r.nj))
+                continue;
+            r.form = LV_TWO_PASS_F32;
+            v.*run = r;
+            scratch = std::max(scratch, f32_scratch(r, v.P));
+        }
+        return scratch;
+    };
+    p->scratch = p->least_scratch = float32_levels(&DevLevel::run, std::max(f16, Y_BYTES));
+    if (base + align256(f16) <= FFBP_STATIC_WS_BYTES && base + align256(p->scratch) > FFBP_STATIC_WS_BYTES)
+        p->least_scratch = float32_levels(&DevLevel::least, FFBP_STATIC_WS_BYTES - base);
+    else
+        for (auto &v : p->lv) v.least = v.run;
 }
 
 const char *const WAIT_MSG = "a tensor-core kernel stopped waiting on its pipeline (a bounded wait ran out) and "
@@ -300,6 +329,43 @@ int aborted(ffbp_plan *p, const char *when)
 }
 
 }  // namespace
+
+namespace ffbp {
+// The bytes of the smallest workspace a form call takes (ffbp_plan_workspace_bytes names the one it is fastest on).
+size_t plan_least_workspace(const ffbp_plan *p)
+{
+    return 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2)) + align256(p->least_scratch);
+}
+}  // namespace ffbp
+
+// A level in two passes through a float32 intermediate, a launch pair at a time (LevelRun); mark after each launch.
+template <class Mark>
+static cudaError_t two_pass_f32(const ffbp::LevelLaunch &L, const LevelRun &r, const int *amax_in, void *scratch, int *err,
+                                cudaStream_t s, const char **why, Mark mark)
+{
+    for (int n0 = 0; n0 < L.Np; n0 += r.nn)
+        for (int c0 = 0; c0 < L.C; c0 += r.nc)
+            for (int j0 = 0; j0 < L.Ko; j0 += r.nj) {
+                ffbp::LevelLaunch A = L;
+                int n = n0;
+                const int nn = std::min(r.nn, L.Np - n0), nj = std::min(r.nj, L.Ko - j0);
+                if (r.nc < L.C) {                        // some of one parent's children: a level of their own
+                    A.x += (size_t)n0 * L.P * L.K;
+                    A.phase += ((size_t)n0 * L.C + c0) * L.P;
+                    A.out += ((size_t)n0 * L.C + c0) * L.Po * L.Ko;
+                    A.Np = 1;
+                    A.C = std::min(r.nc, L.C - c0);
+                    n = 0;
+                }
+                cudaError_t e = ffbp::launch_level_mma(A, amax_in, scratch, false, n, nn, j0, nj, err, s, why);
+                if (*why || e != cudaSuccess) return e;
+                mark(FFBP_KIND_LEVEL_TC_GEMM);
+                e = ffbp::launch_level_fir32(A, amax_in, scratch, n, nn, j0, nj, s, why);
+                if (*why || e != cudaSuccess) return e;
+                mark(FFBP_KIND_LEVEL_TC_FIR);
+            }
+    return cudaSuccess;
+}
 
 extern "C" {
 
@@ -506,7 +572,8 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     if (int rc = aborted(p, "an earlier form call on this plan")) return rc;
     size_t need;
     ffbp_plan_workspace_bytes(p, &need);
-    if (ws_bytes < need) return fail(FFBP_E_WORKSPACE, "workspace of %zu bytes, %zu needed", ws_bytes, need);
+    if (ws_bytes < ffbp::plan_least_workspace(p)) return fail(FFBP_E_WORKSPACE, "workspace of %zu bytes, %zu needed", ws_bytes, need);
+    LevelRun DevLevel::*const run = ws_bytes >= need ? &DevLevel::run : &DevLevel::least;
     if (((uintptr_t)d_ws & 255) != 0) return fail(FFBP_E_ARG, "workspace must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream_);
     char *ws = static_cast<char *>(d_ws);
@@ -531,12 +598,13 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     };
     mark(0);
     const float2 *in = static_cast<const float2 *>(d_S);
-    if (two_pass(p->lv[0])) {
+    if (two_pass(p->lv[0].*run)) {
         if ((e = ffbp::launch_amax(in, (size_t)p->lv[0].P * p->lv[0].K, amax, s)) != cudaSuccess) return cuda_fail(e, "history scan");
         mark(FFBP_KIND_AMAX << 8);
     }
     for (int l = 0; l < p->nlev; ++l) {
         const DevLevel &v = p->lv[l];
+        const LevelRun &r = v.*run;
         float2 *outp = (l % 2 == 0) ? bufA : bufB;
         ffbp::LevelLaunch L;
         L.x = in; L.phase = v.phase; L.tk = v.tk; L.tp = v.tp;
@@ -550,13 +618,13 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
         L.tc_nt = v.tc.nt; L.tc_sb = v.tc.sb; L.tc_pc = v.tc.copies; L.tc_rp = v.tc.repeat; L.tc_fir = v.tc.fir;
         L.tc_cw = v.tc.consumers;
         const char *why = nullptr;
-        if (v.form == LV_ONE_PASS) {
+        if (r.form == LV_ONE_PASS) {
             e = ffbp::launch_level_fused(L, p->d_aborts, s, &why);
             if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC << 8 | l);
-        } else if (v.form == LV_FP32) {
+        } else if (r.form == LV_FP32) {
             e = ffbp::launch_level(L, s, &why);
             if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL << 8 | l);
-        } else if (v.form == LV_TWO_PASS_F16) {
+        } else if (r.form == LV_TWO_PASS_F16) {
             e = ffbp::launch_level_tc_gemm(L, amax + l, scratch, p->d_aborts, s, &why);
             if (!why && e == cudaSuccess) {
                 mark(FFBP_KIND_LEVEL_TC_GEMM << 8 | l);
@@ -564,15 +632,7 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
                 if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC_FIR << 8 | l);
             }
         } else {
-            for (int n0 = 0; n0 < v.Np && !why && e == cudaSuccess; n0 += v.nn)
-                for (int j0 = 0; j0 < v.Ko && !why && e == cudaSuccess; j0 += v.nj) {
-                    const int nn = std::min(v.nn, v.Np - n0), nj = std::min(v.nj, v.Ko - j0);
-                    e = ffbp::launch_level_mma(L, amax + l, scratch, false, n0, nn, j0, nj, p->d_aborts, s, &why);
-                    if (why || e != cudaSuccess) break;
-                    mark(FFBP_KIND_LEVEL_TC_GEMM << 8 | l);
-                    e = ffbp::launch_level_fir32(L, amax + l, scratch, n0, nn, j0, nj, s, &why);
-                    if (!why && e == cudaSuccess) mark(FFBP_KIND_LEVEL_TC_FIR << 8 | l);
-                }
+            e = two_pass_f32(L, r, amax + l, scratch, p->d_aborts, s, &why, [&](int kind) { mark(kind << 8 | l); });
         }
         if (why) return fail(FFBP_E_UNSUPPORTED, "level %d: %s", l, why);
         if (e != cudaSuccess) return cuda_fail(e, "level kernel");
@@ -908,9 +968,11 @@ int ffbp_plan_info(const ffbp_plan *p, int *nlev, int *launches)
     if (nlev) *nlev = p->nlev;
     if (launches) {
         int n = 1;
-        for (const auto &v : p->lv)
-            n += two_pass(v) ? 2 * ((v.Np + v.nn - 1) / v.nn) * ((v.Ko + v.nj - 1) / v.nj) : 1;
-        if (two_pass(p->lv[0])) n += 1;                            // the history scan
+        for (const auto &v : p->lv) {
+            const LevelRun &r = v.run;
+            n += two_pass(r) ? 2 * ((v.Np + r.nn - 1) / r.nn) * ((v.C + r.nc - 1) / r.nc) * ((v.Ko + r.nj - 1) / r.nj) : 1;
+        }
+        if (two_pass(p->lv[0].run)) n += 1;                        // the history scan
         *launches = n;
     }
     return FFBP_OK;

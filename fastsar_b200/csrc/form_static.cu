@@ -4,7 +4,8 @@
 // Who needs it: a caller that cannot allocate device memory at the time it forms an image -- a process whose
 // device memory is handed out by a pool it does not control, a real-time loop that must not enter the CUDA
 // allocator (cudaMalloc can synchronise the device and take milliseconds), or code running where no allocator is
-// reachable. Such a caller builds its plan during set-up and then forms images of plans whose workspace fits here.
+// reachable. Such a caller builds its plan during set-up and then forms images of plans whose least workspace fits here
+// (the float32 form's intermediates take what is left of it, in more launches than ffbp_form's on a whole workspace).
 //
 // The scratch is g_static_ws below, FFBP_STATIC_WS_BYTES (64 MiB): every GPU that loads this library holds it
 // until the process exits. Host code only sees a stand-in for that array, not a device address, so its device
@@ -23,6 +24,7 @@ struct ffbp_plan;
 
 namespace ffbp {
 int form_on_workspace(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, size_t ws_bytes, void *stream, int *h_bad);
+size_t plan_least_workspace(const ffbp_plan *p);
 int set_error(int code, const char *msg);
 }  // namespace ffbp
 
@@ -58,12 +60,11 @@ int static_workspace(void **out)
 extern "C" int ffbp_form_static(ffbp_plan *plan, const void *d_S, void *d_img, void *stream, int *h_bad_pulse)
 {
     if (!plan || !d_S || !d_img) return ffbp::set_error(FFBP_E_ARG, "ffbp_form_static: null argument");
-    size_t need = 0;
-    int rc = ffbp_plan_workspace_bytes(plan, &need);
-    if (rc != FFBP_OK) return rc;
+    const size_t need = ffbp::plan_least_workspace(plan);
+    int rc = FFBP_OK;
     if (need > (size_t)FFBP_STATIC_WS_BYTES) {
         char msg[256];
-        snprintf(msg, sizeof msg, "ffbp_form_static: the plan needs %zu bytes of workspace, more than the %zu of the "
+        snprintf(msg, sizeof msg, "ffbp_form_static: the plan needs %zu bytes of workspace at least, more than the %zu of the "
                  "static workspace; use ffbp_form with a workspace of ffbp_plan_workspace_bytes", need,
                  (size_t)FFBP_STATIC_WS_BYTES);
         return ffbp::set_error(FFBP_E_WORKSPACE, msg);

@@ -201,8 +201,9 @@ int ffbp_batch_destroy(ffbp_batch *batch);
 /* ffbp_form without a caller-allocated workspace, for callers that cannot allocate device memory when they form an
  * image (a device pool they do not control, a real-time loop that must not enter the CUDA allocator). No counterpart
  * in the reference. The scratch is a static device array of this library, FFBP_STATIC_WS_BYTES (64 MiB), held by
- * every GPU that loads the library until the process exits; a plan whose ffbp_plan_workspace_bytes exceeds it is
- * rejected with FFBP_E_WORKSPACE. The call allocates nothing. Its first call on a device looks the array's device
+ * every GPU that loads the library until the process exits. A plan whose ffbp_plan_workspace_bytes exceeds it runs its
+ * float32 levels in more and smaller launches where its level outputs (and float16 intermediate) fit, and is rejected
+ * with FFBP_E_WORKSPACE where they do not. The call allocates nothing. Its first call on a device looks the array's device
  * address up (cudaGetSymbolAddress, with that device current), so make that first call before any stream capture.
  * All calls share the array: calls whose work overlaps on the GPU race and must not be made.                    */
 #define FFBP_STATIC_WS_BYTES (64u << 20)

@@ -65,6 +65,38 @@ def test_static_workspace_tensor_core_form(golden):
         assert np.array_equal(img.cpu().numpy().view(np.uint32), ref.view(np.uint32))
 
 
+@pytest.mark.parametrize('n,T', [(768, 32), (1024, 16)])
+def test_static_workspace_takes_what_the_outputs_leave(oracle_lib, n, T):
+    """float32 images whose level outputs fit the static array, but not with a level's whole intermediate: ffbp_form runs
+    every level in one launch pair on the tensor cores, ffbp_form_static in several (columns of the first level's children,
+    8 children and 128 columns at a time at 1,024 pixels; parents of the later ones). The same sums, tiled anew, so that
+    only where the output ramps start and the tensor core's order differ: each image below 1e-5 of the float64 oracle's
+    (as the other float32 images), the two below 2e-6 apart."""
+    from fastsar_b200 import ImageFormer, sim
+    P = 2 * n
+    col = sim.spotlight(P, P, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    e1, e2 = (0.0, 1.0, 0.0), (1.0, 0.0, 0.0)
+    f = ImageFormer(col.ant, col.fmin, col.df, P, n, n, 0.25, 0.25, e1, e2, T=T)
+    assert f._dev.ws_bytes > 64 << 20
+    gen = torch.Generator(device='cuda').manual_seed(n)
+    S = torch.randn((P, P), dtype=torch.complex64, device='cuda', generator=gen)
+    img = torch.empty((n, n), dtype=torch.complex64, device='cuda')
+    kinds = [k for k, _, _ in f._dev.form_profile(S, img)]
+    assert kinds == ['amax'] + ['level_tc_gemm', 'level_tc_fir'] * 3 + ['final_tc'], kinds
+    a = f.form_device(S).cpu().numpy().astype(complex)
+    assert _form_static(f._dev, S, img) == -1
+    b = img.cpu().numpy().astype(complex)
+    form, _ = oracle_lib.image_former(col.ant, col.fmin, col.df, P, n, n, 0.25, 0.25, e1=e1, e2=e2, T=T, kind='port')
+    want = form(S.cpu().numpy())
+
+    def rel(x, y):
+        return np.linalg.norm(x - y) / np.linalg.norm(y)
+    print(f'{n} pixels, T {T}: form {rel(a, want):.1e}, static {rel(b, want):.1e}, apart {rel(b, a):.1e}')
+    assert rel(a, want) < 1e-5 and rel(b, want) < 1e-5 and rel(b, a) < 2e-6
+    S[17, 3] = complex(np.inf, 0.0)
+    assert _form_static(f._dev, S, img) == 17
+
+
 def test_static_workspace_refuses_a_large_plan():
     from fastsar_b200 import ImageFormer, sim
     w = sim.workload('spotlight_4k')
