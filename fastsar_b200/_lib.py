@@ -23,6 +23,7 @@ FFBP_FINAL_CORES = 0x400
 
 # every symbol include/ffbp_b200.h declares
 EXPORTS = ('ffbp_last_error', 'ffbp_abi_version', 'ffbp_plan_create', 'ffbp_plan_destroy', 'ffbp_plan_workspace_bytes',
+           'ffbp_plan_least_workspace_bytes',
            'ffbp_form', 'ffbp_form_timed', 'ffbp_plan_info', 'ffbp_level', 'ffbp_phases', 'ffbp_final',
            'ffbp_bp_points_f64', 'ffbp_bp_pad', 'ffbp_simulate', 'ffbp_form_static', 'ffbp_level_tc', 'ffbp_level_tc_scratch_bytes',
            'ffbp_form_profile', 'ffbp_exact_pad', 'ffbp_exact_backproject', 'ffbp_mlp_param_count',
@@ -82,6 +83,7 @@ def load():
     L.ffbp_plan_create.argtypes = [ctypes.POINTER(PlanDesc), _vp, ctypes.POINTER(_vp)]
     L.ffbp_plan_destroy.argtypes = [_vp]
     L.ffbp_plan_workspace_bytes.argtypes = [_vp, ctypes.POINTER(ctypes.c_size_t)]
+    L.ffbp_plan_least_workspace_bytes.argtypes = [_vp, ctypes.POINTER(ctypes.c_size_t)]
     L.ffbp_form.argtypes = [_vp, _vp, _vp, _vp, ctypes.c_size_t, _vp, ctypes.POINTER(_c_int)]
     L.ffbp_form_static.argtypes = [_vp, _vp, _vp, _vp, ctypes.POINTER(_c_int)]
     L.ffbp_plan_check.argtypes = [_vp, _vp]

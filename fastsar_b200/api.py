@@ -182,20 +182,29 @@ class DevicePlan:
         self.handle = h
         n = ctypes.c_size_t()
         _lib.check(L.ffbp_plan_workspace_bytes(h, ctypes.byref(n)), 'ffbp_plan_workspace_bytes')
-        self.ws_bytes = int(n.value)
+        self.ws_bytes = self._ws_whole = int(n.value)
+        _lib.check(L.ffbp_plan_least_workspace_bytes(h, ctypes.byref(n)), 'ffbp_plan_least_workspace_bytes')
+        self._ws_least = int(n.value)
         self._ws = None
         self._stage = None
 
     def workspace(self):
+        """The address of the workspace, ws_bytes long: the whole one where the device has room for it, else the least
+        (without the float32 form's intermediates, whose levels then run on slower kernels)."""
         import torch
-        if self._ws is None:
+        for size in (self._ws_whole, self._ws_least):
+            if self._ws is not None:
+                break
             try:
-                self._ws = torch.empty(self.ws_bytes + 256, dtype=torch.uint8, device=self.device)
+                self._ws = torch.empty(size + 256, dtype=torch.uint8, device=self.device)
+                self.ws_bytes = size
             except torch.OutOfMemoryError:
+                if size != self._ws_least:
+                    continue
                 free, total = torch.cuda.mem_get_info(self.device)
                 lv = self.plan['levels']
                 raise MemoryError(
-                    f'the plan needs {self.ws_bytes / 2**30:.1f} GiB of device workspace (the levels\' outputs and '
+                    f'the plan needs {size / 2**30:.1f} GiB of device workspace (the levels\' outputs and '
                     f'the tensor-core levels\' float16 intermediate) and {free / 2**30:.1f} of {total / 2**30:.1f} GiB '
                     f'are free on {self.device}; first-level children {lv[0]["C"]}, output samples per level '
                     f'{[l["Ko"] for l in lv]}, pulses {[l["Po"] for l in lv]}. Remedies: a smaller pmax (less '
@@ -207,6 +216,7 @@ class DevicePlan:
 
     def release_workspace(self):
         self._ws = None
+        self.ws_bytes = self._ws_whole
         self._stage = None
 
     def form_host(self, S_ptrs, img_ptrs, stream=None):
@@ -292,7 +302,7 @@ class DevicePlan:
         _lib.check(L.ffbp_form_profile(self.handle, ctypes.c_void_p(S_dev.data_ptr()), ctypes.c_void_p(img_dev.data_ptr()),
                                        ctypes.c_void_p(self.workspace()), ctypes.c_size_t(self.ws_bytes),
                                        ctypes.c_void_p(stream.cuda_stream), ms, kind, n), 'ffbp_form_profile')
-        return [(_lib.KIND_NAMES.get(k >> 8, '?'), k & 0xff, float(m)) for k, m in zip(kind, ms)]
+        return [(_lib.KIND_NAMES.get(k >> 8, '?'), k & 0xff, float(m)) for k, m in zip(kind, ms) if k]
 
     def launches(self):
         """Kernels one form call launches."""

@@ -276,8 +276,9 @@ int window_exponent(const float *wp, int P, const float *wk, int K)
 // through a float32 intermediate where the shape is covered and the phases are small. FFBP_FINAL_TC_F16 with
 // FFBP_LEVELS_TC: in one pass, or with FFBP_LEVELS_TC2 (and for shapes the one-pass kernel does not cover) in two through
 // a float16 intermediate; shapes that form does not cover stay in float32; without it, on the CUDA cores. The least
-// workspace of a plan whose level outputs fit the static workspace fits there too (ffbp_form_static): its float32
-// intermediates take what the outputs leave, in as many launch pairs as that needs. (ffbp_form is not held to that: 1,024 x
+// workspace holds the level outputs and the float16 intermediate, beside which the float32 intermediates take what is left
+// of that intermediate or, where all that fits the static workspace (ffbp_form_static), of the static workspace, in as many
+// launch pairs as that needs; levels of which not even a piece fits run on the CUDA cores. (ffbp_form is not held to that: 1,024 x
 // 1,024 pixels, outputs of 33 MiB and a first intermediate of 132, form in 768 us with it whole, their first level 314.)
 void plan_forms(ffbp_plan *p)
 {
@@ -310,8 +311,8 @@ void plan_forms(ffbp_plan *p)
         return scratch;
     };
     p->scratch = p->least_scratch = float32_levels(&DevLevel::run, std::max(f16, Y_BYTES));
-    if (base + align256(f16) <= FFBP_STATIC_WS_BYTES && base + align256(p->scratch) > FFBP_STATIC_WS_BYTES)
-        p->least_scratch = float32_levels(&DevLevel::least, FFBP_STATIC_WS_BYTES - base);
+    if (base + align256(p->scratch) > FFBP_STATIC_WS_BYTES)
+        p->least_scratch = float32_levels(&DevLevel::least, base + align256(f16) <= FFBP_STATIC_WS_BYTES ? FFBP_STATIC_WS_BYTES - base : f16);
     else
         for (auto &v : p->lv) v.least = v.run;
 }
@@ -529,8 +530,12 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
     // the float32 form: split float16 products on the tensor cores where they cover the shape; with aperture weights,
     // which nothing bounds to float16's range, or where the caller asks for them, the CUDA cores
     p->final_x2 = (d->final_mode & 0xff) == FFBP_FINAL_FP32 && !(d->final_mode & FFBP_FINAL_CORES) && !p->wf && ffbp::final_tc32_supported(p->T, B, p->Pf, p->Qf);
+    if (p->final_x2 && (e = p->alloc(&p->seeds, 2 * (size_t)B * d->Pf)) != cudaSuccess) {
+        if (e != cudaErrorMemoryAllocation) return cleanup(cuda_fail(e, "allocate final seeds"));
+        cudaGetLastError();                              // no room for the seeds: the CUDA cores need none
+        p->final_x2 = false;
+    }
     if (p->final_x2) {
-        if ((e = p->alloc(&p->seeds, 2 * (size_t)B * d->Pf)) != cudaSuccess) return cleanup(cuda_fail(e, "allocate final seeds"));
         e = ffbp::launch_final_seeds2(p->ux, p->uy, (long)B * d->Pf, p->spx, p->spy, p->a0, p->a1, p->seeds, s);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "final seeds kernel"));
     }
@@ -548,6 +553,13 @@ int ffbp_plan_workspace_bytes(const ffbp_plan *p, size_t *bytes)
 {
     if (!p || !bytes) return fail(FFBP_E_ARG, "null argument");
     *bytes = 256 + align256(p->bufA * sizeof(float2)) + align256(p->bufB * sizeof(float2)) + align256(p->scratch);
+    return FFBP_OK;
+}
+
+int ffbp_plan_least_workspace_bytes(const ffbp_plan *p, size_t *bytes)
+{
+    if (!p || !bytes) return fail(FFBP_E_ARG, "null argument");
+    *bytes = ffbp::plan_least_workspace(p);
     return FFBP_OK;
 }
 

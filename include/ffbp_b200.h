@@ -34,7 +34,7 @@ enum {
     FFBP_E_ARG = -1,        /* an argument is out of range (the message names it)                         */
     FFBP_E_CUDA = -2,       /* a CUDA call failed                                                           */
     FFBP_E_NOMEM = -3,      /* a device allocation of the plan failed                                       */
-    FFBP_E_WORKSPACE = -4,  /* the workspace passed to ffbp_form is smaller than ffbp_plan_workspace_bytes   */
+    FFBP_E_WORKSPACE = -4,  /* the workspace passed to ffbp_form is smaller than the plan's least             */
     FFBP_E_UNSUPPORTED = -5,/* a shape the kernels do not cover (the message says which limit)              */
     FFBP_E_TRANSFER = -6    /* a history did not reach the device as it is in host memory (ffbp_form_host)  */
 };
@@ -137,6 +137,9 @@ int ffbp_plan_destroy(ffbp_plan *plan);
 
 /* Bytes of device workspace a form call needs (the level intermediates and a status word).                     */
 int ffbp_plan_workspace_bytes(const ffbp_plan *plan, size_t *bytes);
+/* The smallest workspace a form call takes: the float32 form's intermediates (up to 2 GiB) left out or cut down, its
+ * levels on the CUDA cores or in more launches; slower, and rounded differently.                                  */
+int ffbp_plan_least_workspace_bytes(const ffbp_plan *plan, size_t *bytes);
 
 /* Form the image: d_S [P0, K0] complex64 phase history (unwindowed; the plan's window is applied here; aligned to 8
  * bytes, as a complex64 array is) -> d_img [nx, ny] complex64. d_ws: the workspace (ffbp_plan_workspace_bytes, 256-byte aligned). The device the plan

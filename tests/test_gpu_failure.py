@@ -98,6 +98,38 @@ def test_transfer_that_did_not_deliver_is_reported(golden):
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
 
 
+def test_least_workspace_where_the_whole_does_not_fit(monkeypatch):
+    """A device without room for the float32 levels' intermediates forms on the least workspace (the level outputs), as it
+    did on a plan without intermediates: its levels on the CUDA cores, the image the same to that kernel's float32 phases
+    (1e-7 a cycle, up to 170 cycles at the first level and less later: below 3e-5); a former that is released asks for the
+    whole one again."""
+    from fastsar_b200 import ImageFormer, sim
+    w = sim.workload('spotlight_4k')
+    col = w['col']
+    f = ImageFormer(col.ant, col.fmin, col.df, col.K, w['nx'], w['ny'], w['spx'], w['spy'], w['e1'], w['e2'])
+    whole, least = f._dev._ws_whole, f._dev._ws_least
+    outputs = [1.0 * np.prod([l['C'] for l in f._plan['levels'][:k + 1]]) * f._plan['levels'][k]['Po'] *
+               f._plan['levels'][k]['Ko'] * 8 for k in range(3)]
+    assert least < max(outputs[0], outputs[2]) + outputs[1] + 4096 < whole
+    S = torch.randn((col.Np, col.K), dtype=torch.complex64, device='cuda', generator=torch.Generator(device='cuda').manual_seed(5))
+    out = torch.empty((w['nx'], w['ny']), dtype=torch.complex64, device='cuda')
+    want = f.form_device(S).clone()
+    f.release()
+    empty = torch.empty
+
+    def small(n, **kw):
+        if n == whole + 256:
+            raise torch.OutOfMemoryError('the whole workspace')
+        return empty(n, **kw)
+    with monkeypatch.context() as m:
+        m.setattr(torch, 'empty', small)
+        kinds = [k for k, _, _ in f._dev.form_profile(S, out)]
+    assert kinds == ['level_fp32'] * 3 + ['final_tc'] and f._dev.ws_bytes == least, kinds
+    assert float((out - want).norm() / want.norm()) < 3e-5
+    f.release()
+    assert torch.equal(torch.view_as_real(f.form_device(S)), torch.view_as_real(want)) and f._dev.ws_bytes == whole
+
+
 def test_workspace_that_does_not_fit_names_remedies():
     """A plan whose workspace exceeds the device (learned taps at pmax 0.95 on the 4,096-pulse spotlight: the
     Kaiser-sinc fallback's long filters and nearly no decimation ask for hundreds of GiB) raises MemoryError naming
