@@ -31,9 +31,10 @@ def backproject_device(S, ant, fmin, df, points, *, rcv=None, ref=None, upsample
     tx = np.ascontiguousarray(ant, np.float64)
     if ref is None:
         ref = np.linalg.norm(tx, axis=1) if rcv is None else 0.5 * (np.linalg.norm(tx, axis=1) + np.linalg.norm(rcv, axis=1))
-    # complex64 rows, windowed in float32; wider ones stay in float64 without a window
+    # complex64 rows, windowed in float32; wider ones stay in float64 without a window. The kernel reads the buffer: a lazily
+    # conjugated history (S.conj()) is resolved first
     narrow = window or St.dtype in (torch.complex64, torch.float32, torch.float16, torch.bfloat16)
-    St = St.to(torch.complex64 if narrow else torch.complex128).contiguous()
+    St = St.to(torch.complex64 if narrow else torch.complex128).resolve_conj().resolve_neg().contiguous()
     wp = wk = None
     if window:
         from .api import _window

@@ -234,6 +234,28 @@ def test_points_lanes_match_numpy(N, P):
     assert _rel(got, want) < 2e-9
 
 
+@pytest.mark.parametrize('window', [True, False])
+@pytest.mark.parametrize('make', [
+    lambda S: S.conj(),                                    # conjugated when read
+    lambda S: S.T.contiguous().T,                          # pulses the fast axis
+    lambda S: S.to(torch.complex64).conj()[:, ::2],
+    lambda S: S.real,                                      # a real view of complex storage
+    lambda S: torch._neg_view(S.conj()),                   # negated and conjugated when read
+    lambda S: S[:1].expand(9, -1),
+], ids=['conj', 'transposed', 'strided', 'real', 'neg', 'expanded'])
+def test_points_take_any_view_of_a_history(make, window):
+    """backproject_device on views whose buffer is not the history as it reads: the bits of the materialised copy's."""
+    from fastsar_b200.exact import backproject_device
+    gen = torch.Generator(device='cuda').manual_seed(4)
+    S = torch.randn((9, 48), dtype=torch.complex128, device='cuda', generator=gen)
+    v = make(S)
+    ant = np.stack([np.full(9, -7e3), np.linspace(-60, 60, 9), np.full(9, 7e3)], 1)
+    pts = np.random.default_rng(1).uniform(-20, 20, (50, 3))
+    got = backproject_device(v, ant, 9.6e9, 2e6, pts, window=window)
+    want = backproject_device(torch.from_numpy(v.cpu().resolve_conj().resolve_neg().numpy().copy()), ant, 9.6e9, 2e6, pts, window=window)
+    assert torch.equal(torch.view_as_real(got), torch.view_as_real(want))
+
+
 @pytest.mark.parametrize('w1,w2', [(1, 3), (2, 2), (5, 7), (8, 3), (11, 10), (12, 5)])
 @pytest.mark.parametrize('n1,n2', [(7, 5), (67, 250)])
 def test_coherence_windows(n1, n2, w1, w2):
