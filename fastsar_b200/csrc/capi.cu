@@ -1054,6 +1054,33 @@ int ffbp_level_tc_ex(const void *d_x, int Np, int P, int K, const void *d_phase,
     return FFBP_OK;
 }
 
+int ffbp_level_tc32(const void *d_x, int Np, int P, int K, const void *d_phase, int C, const float *d_tk, int Lk, int plk,
+                    int Dk, int Ko, double kc, const float *d_tp, int Lp, int plp, int Dp, int Po, const float *d_wp,
+                    const float *d_wk, void *d_out, int *d_bad, void *d_scratch, size_t scratch_bytes, int *d_status,
+                    void *stream)
+{
+    if (!d_x || !d_phase || !d_out || !d_scratch || !d_status) return fail(FFBP_E_ARG, "ffbp_level_tc32: null buffer");
+    if (Np < 1 || P < 1 || K < 1 || C < 1 || Dk < 1 || Dp < 1 || Ko < 1 || Po < 1) return fail(FFBP_E_ARG, "ffbp_level_tc32: non-positive size");
+    if ((Dk > 1 && (!d_tk || Lk < 1)) || (Dp > 1 && (!d_tp || Lp < 1))) return fail(FFBP_E_ARG, "ffbp_level_tc32: taps missing");
+    if (((uintptr_t)d_scratch & 15) != 0) return fail(FFBP_E_ARG, "ffbp_level_tc32: scratch must be 16-byte aligned");
+    LevelRun r;
+    if (!two_pass_chunk(r, Np, C, P, Ko, scratch_bytes)) return fail(FFBP_E_WORKSPACE, "ffbp_level_tc32: scratch of %zu bytes is too small", scratch_bytes);
+    if (!ffbp::level_mma_supported(r.nc, Dk > 1 ? Lk : 1, Dk, r.nj)) return fail(FFBP_E_UNSUPPORTED, "ffbp_level_tc32: %d frequency taps", Lk);
+    ffbp::LevelLaunch L;
+    L.x = static_cast<const float2 *>(d_x); L.phase = static_cast<const float2 *>(d_phase); L.tk = d_tk; L.tp = d_tp;
+    L.wp = d_wp; L.wk = d_wk; L.out = static_cast<float2 *>(d_out); L.bad = d_bad;
+    L.Np = Np; L.C = C; L.P = P; L.K = K; L.Ko = Ko; L.Po = Po; L.Dk = Dk; L.Lk = Lk; L.plk = plk; L.Dp = Dp;
+    L.Lp = Lp; L.plp = plp; L.kc = kc; L.amax = d_status + 2;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cudaError_t e = ffbp::launch_amax(L.x, (size_t)Np * P * K, d_status + 1, s);
+    if (e != cudaSuccess) return cuda_fail(e, "ffbp_level_tc32");
+    const char *why = nullptr;
+    e = two_pass_f32(L, r, d_status + 1, d_scratch, d_status, s, &why, [](int) {});
+    if (why) return fail(FFBP_E_UNSUPPORTED, "ffbp_level_tc32: %s", why);
+    if (e != cudaSuccess) return cuda_fail(e, "ffbp_level_tc32");
+    return FFBP_OK;
+}
+
 int ffbp_level_fused(const void *d_x, int Np, int P, int K, const void *d_phase, int C, const float *d_tk, int Lk,
                      int plk, int Dk, int Ko, double kc, const float *d_tp, int Lp, int plp, int Dp, int Po,
                      const float *d_wp, const float *d_wk, void *d_out, int *d_bad, int *d_status, void *stream)

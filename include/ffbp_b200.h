@@ -259,6 +259,15 @@ int ffbp_level(const void *d_x, int Np, int P, int K, const void *d_phase, int C
  * filled here), [2] the output's. No counterpart in the reference (its levels run in float32 only).            */
 size_t ffbp_level_tc_scratch_bytes(int Np, int C, int P, int Ko);
 
+/* The same level as the float32 form runs it where its rotation phases are small: the products as above, a float32
+ * intermediate in d_scratch (16-byte aligned), the pulse FIR in float32. As many parents, or else columns or children of one,
+ * at a time as scratch_bytes hold; FFBP_E_WORKSPACE where 8 children's 128 columns of a parent do not fit,
+ * FFBP_E_UNSUPPORTED above 512 frequency taps or 16 output pulses per input pulse. d_status as above.             */
+int ffbp_level_tc32(const void *d_x, int Np, int P, int K, const void *d_phase, int C, const float *d_tk, int Lk, int plk,
+                    int Dk, int Ko, double kc, const float *d_tp, int Lp, int plp, int Dp, int Po, const float *d_wp,
+                    const float *d_wk, void *d_out, int *d_bad, void *d_scratch, size_t scratch_bytes, int *d_status,
+                    void *stream);
+
 /* The same level in one pass (the arithmetic of FFBP_LEVELS_TC without FFBP_LEVELS_TC2): the three bfloat16 products,
  * the ramp and the pulse FIR's running sums (tensor memory) in one kernel; the output written once as complex64. No
  * scratch. C <= 64, Lk <= 96 and ceil(Lp / Dp) <= 8 (FFBP_E_UNSUPPORTED otherwise). d_status: 3 ints, zeroed by the

@@ -14,8 +14,8 @@ if not torch.cuda.is_available():
 from test_gpu_parity import _level_case, _oracle_level_full, _rel, _run_level_tc, lib  # noqa: E402,F401
 
 
-@pytest.mark.parametrize('case', [
-    # Np, P, K, C, Dk, Dp, frequency pass fraction
+# Np, P, K, C, Dk, Dp, frequency pass fraction
+LAYOUTS = [
     (5, 37, 60, 4, 2, 2, 0.6),        # a row needs half of the accumulator's rows: two pulses a unit, the last alone
     (3, 43, 30, 9, 1, 3, 0.6),        # Dk = 1 and 30 columns: four pulses a unit, two groups of 8 child columns
     (2, 21, 44, 8, 3, 2, 0.6),        # 23 columns, 25 taps
@@ -26,7 +26,14 @@ from test_gpu_parity import _level_case, _oracle_level_full, _rel, _run_level_tc
     (1, 30, 900, 40, 9, 3, 0.45),     # a plane of 8 samples and a gathered one, two steps of it (9 taps a phase)
     (2, 26, 640, 12, 10, 4, 0.3),     # two gathered planes
     (1, 20, 1500, 5, 17, 2, 0.2),     # two planes of 8 samples and a gathered one
-], ids=lambda c: 'Np%d-P%d-K%d-C%d-Dk%d-Dp%d' % c[:6])
+]
+
+
+def _layout_id(c):
+    return 'Np%d-P%d-K%d-C%d-Dk%d-Dp%d' % c[:6]
+
+
+@pytest.mark.parametrize('case', LAYOUTS, ids=_layout_id)
 def test_level_layouts_match_oracle(lib, oracle_lib, case):  # noqa: F811
     """The mixed-precision level against the float64 oracle: split float16 products (2^-22) and a float16 intermediate
     (2^-12 rms a sample, averaged by the pulse filter): below 5e-4."""
@@ -37,6 +44,59 @@ def test_level_layouts_match_oracle(lib, oracle_lib, case):  # noqa: F811
     e = _rel(got, _oracle_level_full(oracle_lib, x, c0, sl, fk, fp, Ko, Po, Dk, Dp))
     print(f'level {case} Ko {Ko}: rel {e:.2e}')
     assert st[0] == 0 and e < 5e-4
+
+
+def _level_float64(x, c0, sl, fk, fp, Ko, Po, Dk, Dp):
+    """The level in float64: each child's rotated rows, the frequency FIR, the pulse FIR."""
+    def fir(v, f, D, n):                               # along the last axis; zeros outside
+        if f is None:
+            return v
+        h, L, pl = np.asarray(f['kern'], np.float32).astype(float), f['L'], f['pl']
+        v = np.pad(v, [(0, 0)] * (v.ndim - 1) + [(pl, D * n + L)])
+        return np.lib.stride_tricks.sliding_window_view(v, L, -1)[..., :D * n:D, :] @ h[:L]
+    Np, P, K = x.shape
+    C = c0.shape[1]
+    k = np.arange(K) - (K - 1) / 2.0
+    out = np.empty((Np, C, Po, Ko), complex)
+    for n in range(Np):
+        for c in range(C):
+            z = x[n] * np.exp(2j * np.pi * (c0[n, c].astype(float)[:, None] + sl[n, c].astype(float)[:, None] * k))
+            out[n, c] = fir(fir(z, fk, Dk, Ko).T, fp, Dp, Po).T
+    return out.reshape(Np * C, Po, Ko)
+
+
+@pytest.mark.parametrize('case', LAYOUTS + [
+    (1, 21, 2600, 5, 40, 2, 0.4),     # long filters: a tile of 64 columns or fewer
+    (4, 19, 1100, 12, 2, 3, 0.6),     # several parents, columns and children at a time (below)
+], ids=_layout_id)
+def test_float32_level_layouts(lib, case):  # noqa: F811
+    """The float32 form's level through the same layouts, whole and in the pieces that less scratch leaves (parents; columns
+    of one, the last ones odd; 8 of its children and 128 columns), against float64: split float16 products (2^-22), the
+    hardware sine and cosine (4e-7) and float32 sums, 5e-6 (a missing low part of either operand is 1e-4)."""
+    Np, P, K, C, Dk, Dp, pk = case
+    rng = np.random.default_rng(sum(case[:6]))
+    x, c0, sl, fk, fp, Ko, Po = _level_case(rng, Np, P, K, C, Dk, Dp, pk=pk)
+    want = _level_float64(x, c0, sl, fk, fp, Ko, Po, Dk, Dp)
+    L = lib.load()
+    dx, dph = torch.from_numpy(x).cuda(), torch.from_numpy(np.stack([c0, sl], -1).astype(np.float32)).cuda()
+    tk, tp = (torch.from_numpy(np.asarray(f['kern'], np.float32)).cuda() if f else None for f in (fk, fp))
+    parent, column = C * P * (-(-Ko // 4) * 4) * 8, P * 8
+    least = min(parent, 8 * column * (128 if Ko > 128 else -(-Ko // 4) * 4))
+    args = (dx.data_ptr(), Np, P, K, dph.data_ptr(), C, lib.tptr(tk), fk['L'] if fk else 1, fk['pl'] if fk else 0, Dk, Ko,
+            (K - 1) / 2.0, lib.tptr(tp), fp['L'] if fp else 1, fp['pl'] if fp else 0, Dp, Po, None, None)
+    stream = torch.cuda.current_stream().cuda_stream
+    for size in sorted({Np * parent, min(2, Np) * parent, parent, min(parent, C * column * 128), least}, reverse=True):
+        scratch = torch.empty(size // 4 + 4, dtype=torch.int32, device='cuda')
+        out = torch.full((Np * C, Po, Ko), float('nan'), dtype=torch.complex64, device='cuda')
+        status = torch.zeros(3, dtype=torch.int32, device='cuda')
+        lib.check(L.ffbp_level_tc32(*args, out.data_ptr(), None, scratch.data_ptr(), size, status.data_ptr(), stream), 'level')
+        got, st = out.cpu().numpy(), status.cpu().numpy()
+        e = _rel(got, want)
+        print(f'level {case} Ko {Ko}, scratch {size} of {Np * parent}: rel {e:.2e}')
+        assert st[0] == 0 and e < 5e-6
+        assert st[2:].view(np.float32)[0] == max(abs(got.real).max(), abs(got.imag).max())
+    with pytest.raises(ValueError, match='too small'):
+        lib.check(L.ffbp_level_tc32(*args, out.data_ptr(), None, scratch.data_ptr(), column, status.data_ptr(), stream), 'level')
 
 
 @pytest.mark.parametrize('P,K,nx,ny,T,window', [
@@ -259,8 +319,9 @@ def test_points_take_any_view_of_a_history(make, window):
 @pytest.mark.parametrize('w1,w2', [(1, 3), (2, 2), (5, 7), (8, 3), (11, 10), (12, 5)])
 @pytest.mark.parametrize('n1,n2', [(7, 5), (67, 250)])
 def test_coherence_windows(n1, n2, w1, w2):
-    """The coherence for windows with and without kept rows, images smaller than a window among them, and a strip of
-    zeros (0 there) against float64 window sums: float32 column sums and result, 1e-6."""
+    """The coherence at window and run edges, images smaller than a window among them, against float64 window sums: up to 10
+    column sums, each rounded to float32 and added in float32, and the result's rounding, 2e-6; and exactly 0 inside a strip
+    where one image is zero."""
     from scipy.ndimage import uniform_filter
     from fastsar_b200 import products
     rng = np.random.default_rng(n1 + w1)
@@ -277,3 +338,5 @@ def test_coherence_windows(n1, n2, w1, w2):
     got = products.coherence(a, b, w1, w2)
     zero = mean(np.abs(A) ** 2) < 1e-12
     np.testing.assert_allclose(got[~zero], want[~zero], rtol=0, atol=2e-6)
+    np.testing.assert_array_equal(got[zero], 0.0)
+    assert n2 < 50 or zero.any()
