@@ -301,7 +301,7 @@ void plan_forms(ffbp_plan *p)
             if (!(p->final_mode & FFBP_LEVELS_TC) && ((p->final_mode & 0xff) == FFBP_FINAL_TC_F16 || !(v.cycles <= TC_F32_CYCLES)))
                 continue;
             LevelRun r;
-            if ((v.*run).form != LV_FP32 || (Lp + v.Dp - 1) / v.Dp > 16 || !two_pass_chunk(r, v.Np, v.C, v.P, v.Ko, limit) ||
+            if ((v.*run).form != LV_FP32 || !ffbp::level_fir32_supported(Lp, v.Dp) || !two_pass_chunk(r, v.Np, v.C, v.P, v.Ko, limit) ||
                 !ffbp::level_mma_supported(r.nc, Lk, v.Dk, r.nj))
                 continue;
             r.form = LV_TWO_PASS_F32;
@@ -1066,6 +1066,7 @@ int ffbp_level_tc32(const void *d_x, int Np, int P, int K, const void *d_phase, 
     LevelRun r;
     if (!two_pass_chunk(r, Np, C, P, Ko, scratch_bytes)) return fail(FFBP_E_WORKSPACE, "ffbp_level_tc32: scratch of %zu bytes is too small", scratch_bytes);
     if (!ffbp::level_mma_supported(r.nc, Dk > 1 ? Lk : 1, Dk, r.nj)) return fail(FFBP_E_UNSUPPORTED, "ffbp_level_tc32: %d frequency taps", Lk);
+    if (!ffbp::level_fir32_supported(Dp > 1 ? Lp : 1, Dp)) return fail(FFBP_E_UNSUPPORTED, "ffbp_level_tc32: %d pulse taps at a decimation of %d", Lp, Dp);
     ffbp::LevelLaunch L;
     L.x = static_cast<const float2 *>(d_x); L.phase = static_cast<const float2 *>(d_phase); L.tk = d_tk; L.tp = d_tp;
     L.wp = d_wp; L.wk = d_wk; L.out = static_cast<float2 *>(d_out); L.bad = d_bad;

@@ -57,6 +57,7 @@ cudaError_t launch_level_fir_tc(const LevelLaunch &L, const int *amax_in, const 
 // nn - 1 and output columns j0 .. j0 + nj - 1 into y [nn, C, P, (nj + 3) & ~3], float16 (half) or float32 complex, and
 // the pulse FIR of such a float32 intermediate into its place in L.out.
 bool level_mma_supported(int C, int Lk, int Dk, int Ko);
+bool level_fir32_supported(int Lp, int Dp);
 cudaError_t launch_level_mma(const LevelLaunch &L, const int *amax_in, void *y, bool half, int n0, int nn, int j0,
                              int nj, int *err, cudaStream_t s, const char **why);
 cudaError_t launch_level_fir32(const LevelLaunch &L, const int *amax_in, const void *y, int n0, int nn, int j0, int nj,

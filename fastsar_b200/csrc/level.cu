@@ -60,21 +60,23 @@ constexpr int PHB = 16;       // input pulses per batch of child phases (and pul
 
 // Dynamic shared memory: the pulse taps by phase b, [Dp][APE] pairs (t, t) with t = tp[Dp s + b] (zero past Lp), and the
 // frequency taps as pairs (for the packed multiply-adds); the next RX input rows, one column a thread; two finished
-// rows ahead of the frequency FIR; two batches of the children's phases and the pulse weights.
-template <int AP, int G, int NT>
+// rows ahead of the frequency FIR; two batches of the children's phases and the pulse weights. Where the pulse taps do not
+// fit (more than about 3,000 pulses to an output of 8 taps each: chips of collections of 10^5 pulses) they stay in global
+// memory (FAR: the block's threads read the same few each pulse).
+template <int AP, int G, int NT, bool FAR>
 __host__ __device__ constexpr size_t level_smem(int Dp, int Lk)
 {
-    return (size_t)Dp * ((AP + 1) & ~1) * 8 + (size_t)((Lk + 1) & ~1) * 8 + (size_t)RX * NT * 8 + (size_t)2 * G * NT * 8 +
+    return (FAR ? 0 : (size_t)Dp * ((AP + 1) & ~1) * 8) + (size_t)((Lk + 1) & ~1) * 8 + (size_t)RX * NT * 8 + (size_t)2 * G * NT * 8 +
            (size_t)2 * PHB * G * 8 + (size_t)2 * PHB * 4;
 }
 
-template <int AP, int G, int NT>
+template <int AP, int G, int NT, bool FAR>
 __global__ void __launch_bounds__(NT, AP <= 10 ? 512 / NT : 1) level_kernel(const LevelArgs a)
 {
     constexpr int APE = (AP + 1) & ~1;
     extern __shared__ __align__(16) float2 smem[];
     float2 *s_tp = smem;
-    float2 *s_tk = s_tp + a.Dp * APE;
+    float2 *s_tk = s_tp + (FAR ? 0 : a.Dp * APE);
     float2 *s_x = s_tk + ((a.Lk + 1) & ~1);
     float2 *s_z = s_x + RX * NT;
     float2 *s_ph = s_z + 2 * G * NT;                      // [2][PHB][G]
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(NT, AP <= 10 ? 512 / NT : 1) level_kernel(cons
     const bool colok = (t < a.NK) && (k >= 0) && (k < a.K);
     const float kf = (float)k - a.kc;                     // exact: |k| < 2^24 and kc is a multiple of 1/2
 
-    for (int r = t; r < a.Dp * APE; r += NT) {
+    for (int r = t; !FAR && r < a.Dp * APE; r += NT) {
         const int b = r / APE, s = r - b * APE;
         const int tap = a.Dp * s + b;
         const float v = (s < AP && tap < a.Lp) ? (a.tp ? a.tp[tap] : 1.f) : 0.f;
@@ -174,6 +176,15 @@ __global__ void __launch_bounds__(NT, AP <= 10 ? 512 / NT : 1) level_kernel(cons
             float2 tb[APE];
 #pragma unroll
             for (int s2 = 0; s2 < APE; s2 += 2) {
+                if (FAR) {
+#pragma unroll
+                    for (int s = s2; s < s2 + 2; ++s) {
+                        const int tap = a.Dp * s + b;
+                        const float f = (s < AP && tap < a.Lp) ? (a.tp ? __ldg(a.tp + tap) : 1.f) : 0.f;
+                        tb[s] = make_float2(f, f);
+                    }
+                    continue;
+                }
                 const float4 q4 = *reinterpret_cast<const float4 *>(&s_tp[b * APE + s2]);
                 tb[s2] = make_float2(q4.x, q4.y);
                 tb[s2 + 1] = make_float2(q4.z, q4.w);
@@ -242,7 +253,9 @@ __global__ void __launch_bounds__(NT, AP <= 10 ? 512 / NT : 1) level_kernel(cons
     }
 }
 
-template <int AP, int G, int NT>
+constexpr size_t LEVEL_SMEM_MAX = 227 * 1024;
+
+template <int AP, int G, int NT, bool FAR = false>
 cudaError_t launch_t(LevelArgs a, cudaStream_t s)
 {
     a.JB = (a.Dk > 1) ? (NT - a.Lk) / a.Dk + 1 : NT;
@@ -262,18 +275,21 @@ cudaError_t launch_t(LevelArgs a, cudaStream_t s)
     a.nseg = (a.Po + a.SEG - 1) / a.SEG;
     const long nblocks = base * a.nseg;
     if (nblocks > 0x7fffffffL) return cudaErrorInvalidValue;
-    const size_t smem = level_smem<AP, G, NT>(a.Dp, a.Lk);
+    const size_t smem = level_smem<AP, G, NT, FAR>(a.Dp, a.Lk);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(level_kernel<AP, G, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(level_kernel<AP, G, NT, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    level_kernel<AP, G, NT><<<(unsigned)nblocks, NT, smem, s>>>(a);
+    level_kernel<AP, G, NT, FAR><<<(unsigned)nblocks, NT, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 template <int G, int NT>
 cudaError_t launch_g(const LevelArgs &a, int ap, cudaStream_t s)
 {
+    const size_t taps = (size_t)a.Dp * ((ap + 1) & ~1) * 8;       // the rest of the shared memory: level_smem
+    if (taps + level_smem<1, G, NT, true>(0, a.Lk) > LEVEL_SMEM_MAX)
+        return ap <= 8 ? launch_t<8, G, NT, true>(a, s) : launch_t<16, G, NT, true>(a, s);
     switch (ap) {
         case 1: return launch_t<1, G, NT>(a, s);
         case 2: return launch_t<2, G, NT>(a, s);
@@ -345,7 +361,7 @@ cudaError_t launch_level(const LevelLaunch &L, cudaStream_t s, const char **why)
     const int G = gsel ? atoi(gsel) : 4;
     cudaError_t e;
     if (wide) e = launch_g<4, 512>(a, apt, s);
-    else if (G == 8) e = launch_g8(a, apt, s);
+    else if (G == 8 && (size_t)a.Dp * apt * 8 < 96 * 1024) e = launch_g8(a, apt, s);
     else e = launch_g<4, 256>(a, apt, s);
     if (e == cudaErrorInvalidValue) *why = "too many level blocks";
     return e;

@@ -161,7 +161,12 @@ cudaError_t launch_fir(FirArgs f, cudaStream_t s)
     f.SEG = (f.Po + nseg - 1) / nseg;
     f.nseg = (f.Po + f.SEG - 1) / f.SEG;
     if (nb > 0x7fffffffL || f.nseg > 65535) return cudaErrorInvalidValue;
-    level_fir<AP, F32><<<dim3((unsigned)nb, (unsigned)f.nseg), 128, (size_t)f.Dp * APP * sizeof(float2), s>>>(f);
+    const size_t smem = (size_t)f.Dp * APP * sizeof(float2);
+    if (smem > 48 * 1024) {                               // 768 pulses to an output and more, of 8 taps each
+        cudaError_t e = cudaFuncSetAttribute(level_fir<AP, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    level_fir<AP, F32><<<dim3((unsigned)nb, (unsigned)f.nseg), 128, smem, s>>>(f);
     return cudaGetLastError();
 }
 
@@ -309,6 +314,12 @@ cudaError_t launch_level_fir_cc(const LevelLaunch &L, const int *amax_in, const 
 {
     *why = nullptr;
     return run_fir<false>(fir_args(L, amax_in, scratch), s, why);
+}
+
+bool level_fir32_supported(int Lp, int Dp)
+{
+    const int AP = (Lp + Dp - 1) / Dp;
+    return AP <= 16 && (size_t)Dp * ((AP + 3) & ~3) * sizeof(float2) <= 227 * 1024;
 }
 
 cudaError_t launch_level_fir32(const LevelLaunch &L, const int *amax_in, const void *y, int n0, int nn, int j0, int nj,

@@ -11,7 +11,8 @@ torch = pytest.importorskip('torch')
 if not torch.cuda.is_available():
     pytest.skip('no CUDA device', allow_module_level=True)
 
-from test_gpu_parity import _level_case, _oracle_level_full, _rel, _run_level_tc, lib  # noqa: E402,F401
+from test_gpu_parity import (_level_case, _oracle_level_full, _rel, _run_level_gpu, _run_level_tc,  # noqa: E402,F401
+                             lib)
 
 
 # Np, P, K, C, Dk, Dp, frequency pass fraction
@@ -97,6 +98,62 @@ def test_float32_level_layouts(lib, case):  # noqa: F811
         assert st[2:].view(np.float32)[0] == max(abs(got.real).max(), abs(got.imag).max())
     with pytest.raises(ValueError, match='too small'):
         lib.check(L.ffbp_level_tc32(*args, out.data_ptr(), None, scratch.data_ptr(), column, status.data_ptr(), stream), 'level')
+
+
+@pytest.mark.parametrize('Dp,pp,form', [
+    (700, 0.4, 'both'),               # pulse taps of 44 KB: the most in the memory a launch has without asking
+    (1351, 0.4, 'both'),              # 84 KB
+    (3300, 0.4, 'both'),              # 206 KB: too much beside the CUDA-core level's rows, whose taps stay in global memory
+    (4000, 0.4, 'cores'),             # 250 KB: the CUDA-core level alone
+    (2400, 0.75, 'cores'),            # 14 taps a phase, 300 KB
+])
+def test_levels_of_long_pulse_filters(lib, Dp, pp, form):  # noqa: F811
+    """Levels that decimate thousands of pulses to one (chips of collections of 10^5 pulses) on both kernels, against
+    float64: as above 5e-6 (sums of some 10^4 products add float32 roundings of about 1e-7 each, averaged)."""
+    rng = np.random.default_rng(Dp)
+    x, c0, sl, fk, fp, Ko, Po = _level_case(rng, 1, 14 * Dp, 21, 3, 1, Dp, pp=pp)
+    want = _level_float64(x, c0, sl, fk, fp, Ko, Po, 1, Dp)
+    e = _rel(_run_level_gpu(lib, x, c0, sl, fk, fp, Ko, Po, 1, Dp), want)
+    print(f'Dp {Dp}, {fp["L"]} taps: CUDA cores {e:.2e}')
+    assert e < 5e-6
+    L = lib.load()
+    P, K, C = x.shape[1], x.shape[2], 3
+    dx, dph = torch.from_numpy(x).cuda(), torch.from_numpy(np.stack([c0, sl], -1).astype(np.float32)).cuda()
+    tp = torch.from_numpy(np.asarray(fp['kern'], np.float32)).cuda()
+    size = C * P * (-(-Ko // 4) * 4) * 8
+    scratch = torch.empty(size // 4, dtype=torch.int32, device='cuda')
+    out = torch.empty((C, Po, Ko), dtype=torch.complex64, device='cuda')
+    status = torch.zeros(3, dtype=torch.int32, device='cuda')
+
+    def run():
+        lib.check(L.ffbp_level_tc32(dx.data_ptr(), 1, P, K, dph.data_ptr(), C, None, 1, 0, 1, Ko, (K - 1) / 2.0, tp.data_ptr(),
+                                    fp['L'], fp['pl'], Dp, Po, None, None, out.data_ptr(), None, scratch.data_ptr(), size,
+                                    status.data_ptr(), torch.cuda.current_stream().cuda_stream), 'ffbp_level_tc32')
+    if form == 'cores':
+        with pytest.raises(ValueError, match='pulse taps'):
+            run()
+        return
+    run()
+    e = _rel(out.cpu().numpy(), want)
+    print(f'Dp {Dp}, {fp["L"]} taps: tensor cores {e:.2e}')
+    assert e < 5e-6 and int(status[0].item()) == 0
+
+
+def test_chip_of_many_pulses(oracle_lib):
+    """A 64-pixel chip of 65,536 pulses, whose first level takes 1,351 pulses to one: the float32 image against the oracle's
+    (1e-5, as the other float32 images)."""
+    from fastsar_b200 import ImageFormer, sim
+    P, K, n = 65536, 96, 64
+    col = sim.spotlight(P, K, 9.6e9, 300e6, 600e3, 45.0, 1.5)
+    f = ImageFormer(col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, (0.0, 1.0, 0.0), (1.0, 0.0, 0.0), T=16)
+    assert max(l['Dp'] for l in f._plan['levels']) > 1000
+    rng = np.random.default_rng(6)
+    S = (rng.standard_normal((P, K)) + 1j * rng.standard_normal((P, K))).astype(np.complex64)
+    form, _ = oracle_lib.image_former(col.ant, col.fmin, col.df, K, n, n, 0.25, 0.25, e1=(0.0, 1.0, 0.0),
+                                      e2=(1.0, 0.0, 0.0), T=16, kind='port')
+    e = _rel(f(S), form(S))
+    print(f'{P} pulses: rel {e:.2e}')
+    assert e < 1e-5
 
 
 @pytest.mark.parametrize('P,K,nx,ny,T,window', [
