@@ -362,7 +362,7 @@ cudaError_t launch_box_mean(const void *in, int kind, int n1, int n2, int w, int
 cudaError_t launch_coherence(const float2 *a, const float2 *b, int n1, int n2, int w1, int w2, float *out,
                              cudaStream_t s)
 {
-    const int oc = COH_NT - (w2 - 1), rows = w1 <= 8 ? 48 : 64;
+    const int oc = COH_NT - (w2 - 1), rows = w1 <= 8 && n1 <= 48 * 65535 ? 48 : 64;   // at most 65,535 runs a launch
     const dim3 grid((n2 + oc - 1) / oc, (n1 + rows - 1) / rows);
     coherence_kernel<<<grid, COH_NT, 0, s>>>(a, b, n1, n2, w1, w2, rows, out);
     return cudaGetLastError();

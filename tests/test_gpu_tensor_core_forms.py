@@ -397,3 +397,21 @@ def test_coherence_windows(n1, n2, w1, w2):
     np.testing.assert_allclose(got[~zero], want[~zero], rtol=0, atol=2e-6)
     np.testing.assert_array_equal(got[zero], 0.0)
     assert n2 < 50 or zero.any()
+
+
+def test_coherence_of_the_longest_images():
+    """More rows than 65,535 runs of 48 hold: the middle and the last rows against float64 window sums, as above."""
+    from fastsar_b200 import products
+    n1, n2 = 48 * 65535 + 1000, 2
+    gen = torch.Generator(device='cuda').manual_seed(7)
+    a = torch.randn((n1, n2), dtype=torch.complex64, device='cuda', generator=gen)
+    b = a + torch.randn((n1, n2), dtype=torch.complex64, device='cuda', generator=gen)
+    got = products.coherence(a, b, 3, 2)
+    for r in (n1 // 2, n1 - 500):
+        A, B = (v[r - 1:r + 500].to(torch.complex128) for v in (a, b))
+
+        def window(v):                                        # rows i - 1 .. i + 1, columns j - 1 .. j, the edges repeated
+            v = v[:-2] + v[1:-1] + v[2:]
+            return torch.stack([2 * v[:, 0], v[:, 0] + v[:, 1]], 1)
+        want = window(A * B.conj()).abs() / (window(A.abs() ** 2) * window(B.abs() ** 2)).sqrt()
+        assert float((got[r:r + len(want)] - want).abs().max()) < 2e-6
