@@ -232,7 +232,7 @@ bool two_pass_chunk(LevelRun &r, int Np, int C, int P, int Ko, size_t limit)
 }
 
 // The largest rotation phase of a level, in cycles at the edge of its band, over the children of the first, middle and
-// last parent seen from the first, middle and last pulse.
+// last parent seen from the first, middle and last pulse (a sample that a kernel is chosen by, not a bound).
 double level_cycles(const ffbp_level_desc &L, int B, double kc)
 {
     const int ns[3] = {0, B / 2, B - 1}, ps[3] = {0, L.P / 2, L.P - 1};

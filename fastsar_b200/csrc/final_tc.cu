@@ -22,7 +22,7 @@
 //                         kernel it replaces (images 1.4e-6 to 2.1e-6 against 1.5e-6 to 8.8e-6): the ramps' seeds
 //                         come from the plan as hi + lo, their steps are computed to float32's rounding by the loader
 //                         warp, and the accumulations are cut into short segments (the tensor core's sums truncate).
-//                         4,096 tiles of 40 x 46: 533 us (CUDA cores 1,714); 107,520 of 44 x 88: 24.8 ms (83.9);
+//                         4,096 tiles of 40 x 46: 533 us (CUDA cores 1,714); 107,520 of 44 x 88: 23.8 ms (83.9);
 //                         4,320 of 48 x 97 at T = 16: 714 us (2,057). The producers' conversions bound it.
 //   FFBP_FINAL_TC_F16     two T = 32 tiles in float16, A' = [A_1; A_2], B' = [B_1; B_2]: the two diagonal blocks of the
 //                         product are the tiles; or four T = 16 tiles, the four diagonal blocks, each epilogue warp
@@ -1125,7 +1125,7 @@ bool tc_shape(int op, bool weighted, int T, int Pf, int Qf, size_t maxsmem, TcSh
 {
     const bool split = op != OP_F16;
     if (T != 32 && (T != 16 || op == OP_BF16X2)) {
-        *why = "the tensor-core final stage takes T = 32 (split bfloat16 or float16) or T = 16 (float16)";
+        *why = "the tensor-core final stage takes T = 32, or T = 16 (float16 or split float16)";
         return false;
     }
     // warp items per stage: (tile slots) x (A, B) x (pairs of 8-sample groups) over the NPW producer warps

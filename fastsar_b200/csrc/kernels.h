@@ -22,17 +22,17 @@ struct LevelLaunch {
                           // or below 1/4, by which a windowed sample's scale is reduced; 0 for ordinary windows
     unsigned test_wait_ns = 0;   // tensor-core pass 1 only, for tests of the failure report: when nonzero the MMA
                                  // issuer first waits this long on a barrier nothing completes, as a stuck pipeline
-    // tensor-core pass 1 launch options (0: the default): output columns per tile, B stages, plane copies (2 or 4),
-    // row repeat (1: off), consumer warps (8, 4 or 12, 16 less them copying Hankel rows); pass 2's kernel (1: CUDA
-    // cores, 2: tensor cores)
+    // launch options (0: the default): pass 2's kernel (tc_fir; 1: CUDA cores, 2: tensor cores); the others are checked as
+    // an earlier pass 1 took them (output columns per tile, B stages, plane copies, row repeat, consumer warps) and
+    // change nothing
     int tc_nt = 0, tc_sb = 0, tc_pc = 0, tc_rp = 0, tc_fir = 0, tc_cw = 0;
 };
 
 // Returns cudaSuccess, or an error with *why set to a static message for shapes the kernels do not cover.
 cudaError_t launch_level(const LevelLaunch &L, cudaStream_t s, const char **why);
 
-// A level on the tensor cores (level_tc.cu): the frequency FIR of every child as one product per pulse (bfloat16
-// x 3, float32 accumulation) into a float16 intermediate in `scratch` (level_tc_scratch_bytes), then the pulse FIR
+// A level on the tensor cores (level_tc.cu): the frequency FIR of every child as one product per pulse (split float16,
+// float32 accumulation) into a float16 intermediate in `scratch` (level_tc_scratch_bytes), then the pulse FIR
 // in float32. amax_in: the largest |component| of L.x (float bits), which sets the intermediate's scale; L.amax
 // receives the output's. err: raised (atomicAdd) when a bounded wait runs out.
 bool level_tc_supported(int C, int Lk, int Dk);
