@@ -129,7 +129,7 @@ struct ffbp_plan {
     float *wp = nullptr, *wk = nullptr, *wf = nullptr;
     double *ux = nullptr, *uy = nullptr, *ucx = nullptr, *ucy = nullptr, *rc = nullptr;
     float4 *seeds = nullptr;          // the tensor-core final stage's ramp seeds [ntiles, Pf], two each in split float16
-    int wexp = 0;                     // the window's power of two (window_exponent)
+    int wexp = 0, wfexp = 0;          // the powers of two of the window and of the aperture weights (scale_exponent)
     bool final_x2 = false;            // the float32 form's final stage in split float16 on the tensor cores
     int2 *first = nullptr;
     size_t bufA = 0, bufB = 0;
@@ -256,6 +256,14 @@ double level_cycles(const ffbp_level_desc &L, int B, double kc)
 // cycles, 1.8e-5 at 195, 2.7e-5 at 317, 1.2e-4 at 1,870), and a plan's image is to stay what it was to 2e-5.
 constexpr double TC_F32_CYCLES = 170.0;
 
+// The power of two of a largest weight m, 0 where m lies between lo and hi.
+int scale_exponent(double m, double lo, double hi)
+{
+    int ex = 0;
+    if (m > 0.0 && std::isfinite(m) && (m > hi || m < lo)) std::frexp(m, &ex);
+    return ex;
+}
+
 // The power of two of the window's largest product where that is far from one (LevelLaunch::wexp): the first level's scale
 // comes from the history's largest sample before the window, and leaves float16's range room for a few powers of two only.
 // Ordinary windows (a Taylor window of sum P: 2.8) are left as they are.
@@ -266,10 +274,7 @@ int window_exponent(const float *wp, int P, const float *wk, int K)
         for (int i = 0; w && i < n; ++i) m = std::max(m, std::fabs((double)w[i]));
         return w ? m : 1.0;
     };
-    const double m = wp ? most(wp, P) * most(wk, K) : 1.0;
-    int ex = 0;
-    if (m > 0.0 && std::isfinite(m) && (m > 4.0 || m < 0.25)) std::frexp(m, &ex);
-    return ex;
+    return scale_exponent(wp ? most(wp, P) * most(wk, K) : 1.0, 0.25, 4.0);
 }
 
 // How each level runs, and the scratch of the two-pass ones. float32 form (and split bfloat16 final stage): two passes
@@ -509,6 +514,10 @@ int ffbp_plan_create(const ffbp_plan_desc *d, void *stream_, ffbp_plan **out)
         if (d->wf_ndim != 3) return cleanup(fail(FFBP_E_UNSUPPORTED, "aperture weights: pass the [3, ntiles, Pf] form (weight and gradients)"));
         if ((e = upload(d->h_wf, sizeof(float) * 3 * (size_t)B * d->Pf, &q, true)) != cudaSuccess) return cleanup(cuda_fail(e, "upload weights"));
         p->wf = (float *)q;
+        double most = 0.0;                                // over a tile's rows
+        for (size_t i = 0, n = (size_t)B * d->Pf; i < n; ++i)
+            most = std::max(most, std::fabs((double)d->h_wf[i]) + std::fabs((double)d->h_wf[n + i]) * 0.5 * d->T * d->spx);
+        p->wfexp = scale_exponent(most, 1.0 / 64.0, 1.0);
     }
     if ((e = upload(d->h_first_f, sizeof(int) * 2 * (size_t)B, &q, true)) != cudaSuccess) return cleanup(cuda_fail(e, "upload tile origins"));
     p->first = (int2 *)q;
@@ -653,7 +662,7 @@ static int form_impl(ffbp_plan *p, const void *d_S, void *d_img, void *d_ws, siz
     ffbp::FinalLaunch F;
     F.d = in; F.B = p->ntiles; F.Pf = p->Pf; F.Qf = p->Qf; F.T = p->T; F.ux = p->ux; F.uy = p->uy; F.seeds = p->seeds;
     F.spx = p->spx; F.spy = p->spy; F.a0 = p->a0; F.a1 = p->a1; F.fc2 = p->fc2; F.ucx = p->ucx; F.ucy = p->ucy;
-    F.rc = p->rc; F.w = p->wf; F.tiles = nullptr; F.img = static_cast<float2 *>(d_img); F.first = p->first;
+    F.rc = p->rc; F.w = p->wf; F.wexp = p->wfexp; F.tiles = nullptr; F.img = static_cast<float2 *>(d_img); F.first = p->first;
     F.nx = p->nx; F.ny = p->ny; F.ox = p->ox; F.oy = p->oy; F.scale = 1.f; F.err = p->d_aborts;
     F.amax = amax + p->nlev;
     F.test_wait_ns = p->test_kind == FFBP_KIND_FINAL_TC ? p->test_ns : 0u;

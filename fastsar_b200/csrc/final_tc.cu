@@ -192,6 +192,7 @@ struct TcArgs {
     float scale;
     int *err;
     const int *amax;
+    int wexp;                              // the weights' power of two (FinalLaunch::wexp)
     int interleave;                        // the order of the producer warps' items (final_tc_kernel)
     int nwi;                               // producer items per stage
     int seg, nsg;                          // final subapertures per accumulation (even unless all), accumulations per unit
@@ -199,15 +200,16 @@ struct TcArgs {
 };
 
 // The power of two s that brings samples whose components are at most *amax (a float's bits; null: unknown) to
-// below 2^13 in magnitude, so that d s times a ramp and a weight stays inside float16's range (65504).
-__device__ __forceinline__ float operand_scale(const int *amax)
+// below 2^13 in magnitude, weighted by at most 2^wexp, so that d s times a ramp and a weight stays inside float16's range
+// (65504).
+__device__ __forceinline__ float operand_scale(const int *amax, int wexp)
 {
     if (!amax) return 1.f;
     const float m = __int_as_float(*amax);
     if (!(m > 0.f) || !isfinite(m)) return 1.f;
     int ex;
     frexpf(m, &ex);                                             // m < 2^ex
-    return ldexpf(1.f, min(max(13 - ex, -120), 120));           // it and its inverse normal float32 numbers
+    return ldexpf(1.f, min(max(13 - ex - wexp, -120), 120));           // it and its inverse normal float32 numbers
 }
 
 // The operands' arithmetic: float16, or x = hi + lo in bfloat16 (16 bits) or in float16 (22 bits).
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
                 } else if (fs) {
                     if (lane == 0) cp_async(gd, (const void *)(a.seeds + bp), 16, tv);
                 } else if (lane < 2) cp_async(gd + 8u * lane, (const void *)((lane ? a.uy : a.ux) + bp), 8, tv);
-                else if (WEIGHTED && lane < 5)
+                if (WEIGHTED && lane >= 2 && lane < 5)
                     cp_async(gd + 16u + 4u * (lane - 2), (const void *)(a.w + (size_t)(lane - 2) * nbp + bp), 4, tv);
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&lfull[ls])) : "memory");
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
 #pragma unroll
             for (int k = 0; k < 4; ++k) roff[k] = (uint32_t)(((rows[k] >> 3) * ng) * 128 + (rows[k] & 7) * 16);
         }
-        const float dscale = operand_scale(a.amax), m = (float)(2 * r - (TT - 1));
+        const float dscale = operand_scale(a.amax, a.wexp), m = (float)(2 * r - (TT - 1));
         const int rs = a.S / nis, turn = (a.nwi + 1) % NPW;
         int ps0 = 0, ps1 = 0, p = 0, first = pw;
         uint32_t pp0 = 0, pp1 = 0;
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
         }
         const float sp32x = (float)a.spx, sp32y = (float)a.spy;
         // the float16 operands carry d scaled by a power of two that keeps them inside the format's range
-        const float dscale = BF ? 1.f : operand_scale(a.amax);
+        const float dscale = BF ? 1.f : operand_scale(a.amax, a.wexp);
         // issuer k's stages are k + nis s for s < S / nis, filled and consumed in that issuer's order (one
         // consumer per stage: no wait can run two phases ahead); (ps_k, pp_k) is issuer k's next slot and parity
         const int rs = a.S / nis;
@@ -857,7 +859,7 @@ __global__ void __launch_bounds__(block_threads<OP, WEIGHTED, MAXWI, TT>(), 1) f
     } else {
         // ------------------------------------------------------------------ epilogue (warps 0..3)
         float *P0 = sP, *P1 = sP + 32 * 65;
-        const float oscale = a.scale / (BF ? 1.f : operand_scale(a.amax));
+        const float oscale = a.scale / (BF ? 1.f : operand_scale(a.amax, a.wexp));
         // after a failed wait a warp keeps stepping through the units (and the epilogue's named barriers, which all
         // four warps must reach) without waiting, reading or writing
         bool live = true;
@@ -1196,7 +1198,7 @@ cudaError_t launch_final_tc(const FinalLaunch &F, int mode, cudaStream_t s, cons
     a.nsg = (F.Pf + a.seg - 1) / a.seg;
     a.ux = F.ux; a.uy = F.uy; a.seeds = F.seeds; a.spx = F.spx; a.spy = F.spy; a.a0 = F.a0; a.a1 = F.a1; a.fc2 = F.fc2;
     a.ucx = F.ucx; a.ucy = F.ucy; a.rc = F.rc; a.w = F.w; a.tiles = F.tiles; a.img = F.img; a.first = F.first;
-    a.nx = F.nx; a.ny = F.ny; a.ox = F.ox; a.oy = F.oy; a.scale = F.scale; a.err = F.err; a.amax = F.amax;
+    a.nx = F.nx; a.ny = F.ny; a.ox = F.ox; a.oy = F.oy; a.scale = F.scale; a.err = F.err; a.amax = F.amax; a.wexp = F.w ? F.wexp : 0;
     a.test_wait_ns = F.test_wait_ns;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);

@@ -92,6 +92,7 @@ struct FinalLaunch {
     int *err = nullptr;   // raised (atomicAdd) by a kernel whose bounded wait ran out (tensor-core stage), or null
     const int *amax = nullptr;   // the largest |component| of d (float bits), for the float16 operands' scale
     unsigned test_wait_ns = 0;   // tensor-core stage only, for tests of the failure report (as in LevelLaunch)
+    int wexp = 0;                    // the power of two of the largest aperture weight where above 1 or below 2^-6
     const float4 *seeds = nullptr;   // [B, Pf] the float16 form's ramp seeds (launch_final_seeds), or null
 };
 cudaError_t launch_final_fp32(const FinalLaunch &F, cudaStream_t s, const char **why);

@@ -31,3 +31,26 @@ def test_aperture_weight_matches_reference_former(golden, oracle_lib, nlev):
     # and the weight matters: the unweighted image is far from the weighted one
     plain = ImageFormer(img['ant'], fmin, df, int(K), 128, 128, 0.5, 0.5, T=16, levels=nlev, window=False)(img['S'])
     assert oracle_lib.err_db(plain, ref) > -30.0
+
+
+@pytest.mark.parametrize('T,scale', [(16, 1.0), (32, 1.0), (16, 1e4), (32, 1e-5)])
+def test_aperture_weight_in_float16(golden, T, scale):
+    """The mixed-precision form with an aperture weight (its final stage seeds its ramps from the plan and weights its
+    operands) against the float32 form with the same weight and filters: a float16 intermediate and operands, 2^-11 a
+    factor, below 2e-3; weights of any scale, twice the same bits."""
+    from fastsar_b200 import ImageFormer
+    img = golden('image_small')
+    fmin, df, K = img['scal']
+    P = img['ant'].shape[0]
+    w = weight_fn(P)
+
+    def former(precision):
+        return ImageFormer(img['ant'], fmin, df, int(K), 128, 128, 0.5, 0.5, T=T, atten=80.0, precision=precision,
+                           aperture_weight=lambda points, pulses: scale * w(points, pulses))
+    want = former('float32')(img['S']).astype(complex)
+    f = former('float16')
+    got = f(img['S'])
+    e = np.linalg.norm(got - want) / np.linalg.norm(want)
+    print(f'float16 with an aperture weight, T {T}, scale {scale:g}: {e:.1e}')
+    assert e < 2e-3
+    assert np.array_equal(got.view(np.uint32), f(img['S']).view(np.uint32))
