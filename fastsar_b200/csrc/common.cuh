@@ -1,6 +1,7 @@
 // Shared helpers of the ffbp_b200 kernels (sm_100a).
 #pragma once
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 namespace ffbp {
@@ -35,17 +36,28 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// 2^e, e in [-126, 127]
+__device__ __forceinline__ float pow2(int e)
+{
+    return __int_as_float((127 + e) << 23);
+}
+
+// ex with 2^(ex - 1) <= m < 2^ex of a largest component m given as its float bits; INT_MIN where m is 0, below the normal
+// numbers or not finite, or there is none. On the bits: every thread of the pulse FIR evaluates it.
+__device__ __forceinline__ int top_exponent(const int *amax)
+{
+    const int b = amax ? *amax : 0;
+    return b >= 0x00800000 && b < 0x7f800000 ? (b >> 23) - 126 : INT_MIN;
+}
+
 // e of the power of two 2^e that a tensor-core level's intermediate is scaled by: values up to 4 m (m the input's largest
 // component; the taps' absolute sum is below 4 for the decimators of any plan) come below 2^13, times the window's 2^wexp
 // (LevelLaunch::wexp): a float16 intermediate then stays in range and keeps 11 significant bits. 2^e, 2^-e and an eighth of
 // either are normal float32 numbers.
 __device__ __forceinline__ int level_exponent(const int *amax, int wexp)
 {
-    const float m = amax ? __int_as_float(*amax) : 0.f;
-    if (!(m > 0.f) || !isfinite(m)) return 0;
-    int ex;
-    frexpf(m, &ex);                                             // m < 2^ex
-    return min(max(11 - ex - wexp, -120), 120);
+    const int ex = top_exponent(amax);
+    return ex == INT_MIN ? 0 : min(max(11 - ex - wexp, -120), 120);
 }
 
 // Two float32 fused multiply-adds in one instruction (sm_100's packed FMA): (a.x b.x + c.x, a.y b.y + c.y), each

@@ -192,11 +192,11 @@ struct TcArgs {
     float scale;
     int *err;
     const int *amax;
-    int wexp;                              // the weights' power of two (FinalLaunch::wexp)
     int interleave;                        // the order of the producer warps' items (final_tc_kernel)
     int nwi;                               // producer items per stage
     int seg, nsg;                          // final subapertures per accumulation (even unless all), accumulations per unit
     unsigned test_wait_ns;                 // tests only: the issuers' wait on a barrier nothing completes (0: none)
+    int wexp;                              // the weights' power of two (FinalLaunch::wexp)
 };
 
 // The power of two s that brings samples whose components are at most *amax (a float's bits; null: unknown) to
@@ -204,12 +204,8 @@ struct TcArgs {
 // (65504).
 __device__ __forceinline__ float operand_scale(const int *amax, int wexp)
 {
-    if (!amax) return 1.f;
-    const float m = __int_as_float(*amax);
-    if (!(m > 0.f) || !isfinite(m)) return 1.f;
-    int ex;
-    frexpf(m, &ex);                                             // m < 2^ex
-    return ldexpf(1.f, min(max(13 - ex - wexp, -120), 120));           // it and its inverse normal float32 numbers
+    const int ex = top_exponent(amax);
+    return ex == INT_MIN ? 1.f : pow2(min(max(13 - ex - wexp, -120), 120));   // it and its inverse normal float32 numbers
 }
 
 // The operands' arithmetic: float16, or x = hi + lo in bfloat16 (16 bits) or in float16 (22 bits).

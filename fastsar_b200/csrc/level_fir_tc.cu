@@ -50,12 +50,12 @@ struct FirTcArgs {
     float2 *out;                      // [rows, Po, Ko]
     int *amax;                        // largest |component| of the output (float bits) or null
     const int *amax_in;
-    int wexp;
     int *err;
     int rows, P, Kop, Ko, Po, Dp, Lp, plp;
     int NC, ncb, nob;                 // complex columns per tile, column tiles, output-pulse tiles
     long ntiles;
     int NQ;                           // 16-byte words per shifted tap copy
+    int wexp;
 };
 
 struct TileGeom {
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(R_NTHR, 1) level_fir_tc_kernel(const FirTcArgs
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (warps 0..3)
-        const float inv = ldexpf(1.f, -level_exponent(a.amax_in, a.wexp));
+        const float inv = pow2(-level_exponent(a.amax_in, a.wexp));
         float vmax = 0.f;
         long t_it = 0;
         for (long ti = blockIdx.x; ti < a.ntiles; ti += gridDim.x, ++t_it) {

@@ -66,7 +66,6 @@ struct MmaArgs {
     const float *__restrict__ wk;     // [K] or null
     int *bad;                         // first non-finite pulse or null
     const int *amax_in;
-    int wexp;                         // the window's power of two (LevelLaunch::wexp)
     void *y;                          // [nn, C, P, Kop] from parent n0, column j0: half2 or float2, times 2^level_exponent
     int *err;
     int n0, C, P, K, Dk, Lk, plk;
@@ -83,6 +82,7 @@ struct MmaArgs {
     long nunits;
     float kc;
     unsigned test_wait_ns;
+    int wexp;                         // the window's power of two (LevelLaunch::wexp)
 };
 
 struct Unit {                         // a unit (parent from n0, child group, column group, PP pulses) and its successor
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
         sH[i] = in ? (a.tk ? a.tk[r] : 1.f) * M_TAP_SCALE : 0.f;
     }
     // the samples' power of two, which the window's table carries too (exact)
-    const float xs = ldexpf(1.f / M_TAP_SCALE, level_exponent(a.amax_in, a.wexp));
+    const float xs = pow2(level_exponent(a.amax_in, a.wexp)) / M_TAP_SCALE;
     if (WIN && a.wtab)
         for (int i = t; i < a.K; i += M_NTHR) sW[i] = (a.wk ? a.wk[i] : 1.f) * xs;
     if (warp == M_MW) {

@@ -29,8 +29,8 @@ struct FirArgs {
     float2 *__restrict__ out;         // [rows, Po, Ko], columns nj of it from this pointer on
     int *amax;
     const int *amax_in;
-    int wexp;
     int rows, P, Kop, nj, Ko, Po, Dp, Lp, plp, SEG, nseg;
+    int wexp;                         // (last: the loads of the others pair up; ahead of them 104 registers, 96 here)
 };
 
 // Two complex samples of the intermediate: 8 bytes of float16 or 16 of float32.
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) level_fir(const FirArgs a)
     if (gid >= (long)a.rows * npair) return;
     const int row = (int)(gid / npair), j = 2 * (int)(gid - (long)row * npair);
     const int seg = blockIdx.y;
-    const float inv = ldexpf(1.f, -level_exponent(a.amax_in, a.wexp));
+    const float inv = pow2(-level_exponent(a.amax_in, a.wexp));
     const int i_s = seg * a.SEG, i_e = min(a.Po, i_s + a.SEG);
     const int g_end = i_e + AP - 1;
     const PT *__restrict__ yr = static_cast<const PT *>(a.y) + ((size_t)row * a.P * a.Kop + j) / 2;   // Kop, j even
