@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(M_NTHR, 1) level_mma_kernel(const MmaArgs a)
         sH[i] = in ? (a.tk ? a.tk[r] : 1.f) * M_TAP_SCALE : 0.f;
     }
     // the samples' power of two, which the window's table carries too (exact)
-    const float xs = pow2(level_exponent(a.amax_in, a.wexp)) / M_TAP_SCALE;
+    const float xs = ldexpf(1.f / M_TAP_SCALE, level_exponent(a.amax_in, WIN ? a.wexp : 0));
     if (WIN && a.wtab)
         for (int i = t; i < a.K; i += M_NTHR) sW[i] = (a.wk ? a.wk[i] : 1.f) * xs;
     if (warp == M_MW) {
